@@ -836,6 +836,7 @@ dg_status dg_plan_autotune(dg_plan *plan, const void *d_frames, int32_t dtype, i
         for (int v : {7, 8})
             if (dg::bin_tiles_fill_gpu(plan->gather, v, n_frames))
                 dg::ensure_bin_tiles(plan->gather, plan->table, v, s);
+        dg::ensure_fl_units(plan->gather, plan->table, s);
         std::vector<double> each;
         const int v = dg::autotune_gather(plan->gather, d_frames, dtype,
                                           int64_t(plan->dim1) * plan->dim2, n_frames, flags, s,
@@ -854,6 +855,10 @@ dg_status dg_plan_variant(dg_plan *plan, int32_t set, int32_t *current, int32_t 
         if (set >= 0 && dg::gather_variant_needs_tiles(set)) {
             DeviceScope scope(plan->device);
             dg::ensure_bin_tiles(plan->gather, plan->table, set, plan->stream);
+        }
+        if (set == 5 || set == 6) {
+            DeviceScope scope(plan->device);
+            dg::ensure_fl_units(plan->gather, plan->table, plan->stream);
         }
         if (set >= 0 && !dg::gather_variant_available(plan->gather, set))
             dg::fail(DG_UNSUPPORTED, "gather mapping " + std::to_string(set) +

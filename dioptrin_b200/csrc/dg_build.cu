@@ -422,7 +422,12 @@ __global__ void k_ps1d_count(Ps1d a, int32_t *__restrict__ count, int32_t *__res
 }
 
 // pyfai_1d::sample (pyfai_1d.rs:208-252) for singular pixel blockIdx.x: 128 x
-// 128 x 4 detector-plane samples counted per radial bin of [r0, r1).
+// 128 x 4 detector-plane samples counted per radial bin of [r0, r1), cut over
+// kSampleSlices CTAs (integer counts, so the order of the adds is free). A
+// sample is two double-double arctangents; one CTA per pixel walked 256 of
+// them per thread, 0.84 ms for the one pixel under a beam, and 64 CTAs
+// 49 us.
+constexpr unsigned kSampleSlices = 64;
 __global__ void k_sample(GeomParams g, int dim2, const int32_t *__restrict__ sing, int n,
                          double r0, double r1, int clamp_low, int32_t *__restrict__ hits) {
     const int N = 128;
@@ -431,7 +436,8 @@ __global__ void k_sample(GeomParams g, int dim2, const int32_t *__restrict__ sin
     int32_t *h = hits + int64_t(blockIdx.x) * n;
     double prow = double(pixel / dim2), pcol = double(pixel % dim2);
     const double a0 = -kPi, a1 = kPi;
-    for (int s = threadIdx.x; s < N * N * 4; s += blockDim.x) {
+    for (int s = int(blockIdx.y * blockDim.x + threadIdx.x); s < N * N * 4;
+         s += int(gridDim.y * blockDim.x)) {
         int row = s / (N * 4), col = (s / 4) % N, o = s & 3;
         double d1 = prow + (double(row) + off[o][0]) / double(N);
         double d2 = pcol + (double(col) + off[o][1]) / double(N);
@@ -461,11 +467,34 @@ __global__ void k_sample_count(const int32_t *__restrict__ sing, int n,
     }
 }
 
-// Fill of the pixel-major contribution list; singular pixels copy their
-// sampled hits (bins ascending, weight hits / 65536).
-__global__ void k_ps1d_fill(Ps1d a, const int64_t *__restrict__ off,
-                            const int32_t *__restrict__ sing_slot,
-                            const int32_t *__restrict__ hits, int32_t *__restrict__ cbin,
+// Entries of each sampled (singular) pixel, bins ascending, weight hits/65536
+// (the sum of hits samples of weight 2^-16, exact): one warp per pixel, 32 bins
+// a step. One thread per pixel inside the fill kernel held the whole launch
+// back by its walk over the bins, and needed a slot number per pixel from the
+// host.
+__global__ void k_hits_fill(const int32_t *__restrict__ sing, int64_t nb,
+                            const int32_t *__restrict__ hits, const int64_t *__restrict__ off,
+                            int32_t *__restrict__ cbin, double *__restrict__ cw,
+                            int32_t *__restrict__ cpix) {
+    const int lane = threadIdx.x;  // 32 threads
+    const int32_t pixel = sing[blockIdx.x];
+    const int32_t *h = hits + int64_t(blockIdx.x) * nb;
+    int64_t o = off[pixel];
+    for (int64_t b0 = 0; b0 < nb; b0 += 32) {
+        const int32_t v = b0 + lane < nb ? h[b0 + lane] : 0;
+        const unsigned any = __ballot_sync(0xffffffffu, v != 0);
+        if (v) {
+            const int64_t k = o + __popc(any & ((1u << lane) - 1u));
+            cbin[k] = int32_t(b0 + lane);
+            cw[k] = double(v) / 65536.0;
+            cpix[k] = pixel;
+        }
+        o += __popc(any);
+    }
+}
+
+// Fill of the pixel-major contribution list (singular pixels: k_hits_fill).
+__global__ void k_ps1d_fill(Ps1d a, const int64_t *__restrict__ off, int32_t *__restrict__ cbin,
                             double *__restrict__ cw, int32_t *__restrict__ cpix, int *overflow) {
     int64_t n = int64_t(a.dim1) * a.dim2;
     int bins[kClipCap * 4];
@@ -473,18 +502,6 @@ __global__ void k_ps1d_fill(Ps1d a, const int64_t *__restrict__ off,
     for (int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; p < n;
          p += int64_t(gridDim.x) * blockDim.x) {
         int64_t o = off[p];
-        int32_t s = sing_slot ? sing_slot[p] : -1;
-        if (s >= 0) {
-            const int32_t *h = hits + int64_t(s) * a.n;
-            for (int b = 0; b < a.n; ++b)
-                if (h[b]) {
-                    cbin[o] = b;
-                    cw[o] = double(h[b]) / 65536.0;
-                    cpix[o] = int32_t(p);
-                    ++o;
-                }
-            continue;
-        }
         // Entries of one pixel are produced in bin order; the local buffer
         // holds a chunk at a time so very wide pixels need no large array.
         int total = int(off[p + 1] - off[p]);
@@ -498,6 +515,7 @@ __global__ void k_ps1d_fill(Ps1d a, const int64_t *__restrict__ off,
         } else {
             // Rare: a pixel spanning more bins than the local buffer. Redo the
             // walk bin by bin (same arithmetic as ps1d_pixel).
+            if (ps1d_pixel<false>(a, p, nullptr, nullptr, overflow) < 0) continue;
             const int64_t w = a.dim2 + 1;
             int64_t b0 = p / a.dim2 * w + p % a.dim2;
             int64_t i00 = b0, i01 = b0 + 1, i11 = b0 + w + 1, i10 = b0 + w;
@@ -658,28 +676,14 @@ __global__ void k_pf1d_count(Pf1d a, int32_t *__restrict__ count, int32_t *__res
     }
 }
 
-__global__ void k_pf1d_fill(Pf1d a, const int64_t *__restrict__ off,
-                            const int32_t *__restrict__ sing_slot,
-                            const int32_t *__restrict__ hits, int32_t *__restrict__ cbin,
+__global__ void k_pf1d_fill(Pf1d a, const int64_t *__restrict__ off, int32_t *__restrict__ cbin,
                             double *__restrict__ cw, int32_t *__restrict__ cpix, int *overflow) {
     const int64_t n = int64_t(a.dim1) * a.dim2;
     int bins[kPfCap];
     double ws[kPfCap];
     for (int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; p < n;
          p += int64_t(gridDim.x) * blockDim.x) {
-        int64_t o = off[p];
-        const int32_t s = sing_slot ? sing_slot[p] : -1;
-        if (s >= 0) {
-            const int32_t *h = hits + int64_t(s) * a.n;
-            for (int b = 0; b < a.n; ++b)
-                if (h[b]) {
-                    cbin[o] = b;
-                    cw[o] = double(h[b]) / 65536.0;
-                    cpix[o] = int32_t(p);
-                    ++o;
-                }
-            continue;
-        }
+        const int64_t o = off[p];
         const int m = pf1d_pixel<true>(a, p, bins, ws, overflow);
         for (int k = 0; k < m; ++k) {
             cbin[o + k] = bins[k];
@@ -1107,7 +1111,8 @@ __global__ void k_sample2d(GeomParams gp, Grid2 g, int dim2, const int32_t *__re
     const int32_t pixel = sing[blockIdx.x];
     int32_t *h = hits + int64_t(blockIdx.x) * g.nr * g.na;
     const int64_t row = pixel / dim2, col = pixel % dim2;
-    for (int sm = threadIdx.x; sm < N * N * 4; sm += blockDim.x) {
+    for (int sm = int(blockIdx.y * blockDim.x + threadIdx.x); sm < N * N * 4;
+         sm += int(gridDim.y * blockDim.x)) {
         const int i = sm / (N * 4), j = (sm / 4) % N, o = sm & 3;
         const double d1 = double(row) + (double(i) + off[o][0]) / double(N);
         const double d2 = (double(col * N + j) + off[o][1]) / double(N);
@@ -1133,25 +1138,6 @@ __global__ void k_sample2d_count(const int32_t *__restrict__ sing, int64_t nb,
         for (int i = 0; i < int(blockDim.x + 31) / 32; ++i) t += wsum[i];
         count[sing[blockIdx.x]] = t;
     }
-}
-
-// Entries of each sampled pixel of a batch, bins ascending, weight hits/65536
-// (the sum of hits samples of weight 2^-16, exact).
-__global__ void k_sample2d_fill(const int32_t *__restrict__ sing, int64_t nb,
-                                const int32_t *__restrict__ hits, const int64_t *__restrict__ off,
-                                int32_t *__restrict__ cbin, double *__restrict__ cw,
-                                int32_t *__restrict__ cpix) {
-    if (threadIdx.x != 0) return;
-    const int32_t pixel = sing[blockIdx.x];
-    const int32_t *h = hits + int64_t(blockIdx.x) * nb;
-    int64_t o = off[pixel];
-    for (int64_t b = 0; b < nb; ++b)
-        if (h[b]) {
-            cbin[o] = int32_t(b);
-            cw[o] = double(h[b]) / 65536.0;
-            cpix[o] = pixel;
-            ++o;
-        }
 }
 
 // build_shared_grid_ss_csr through the exact counted path (supersampled.rs
@@ -1215,19 +1201,34 @@ __global__ void k_chunk_count(const int32_t *__restrict__ cbin, const int32_t *_
     }
 }
 
-// Exclusive scan of every bin's column down the chunks; totals per bin.
-__global__ void k_column_scan(int32_t *__restrict__ m, int n_chunks, int nb,
-                              int64_t *__restrict__ totals) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
+// Exclusive scan of every bin's column down the chunks; totals per bin. A CTA
+// takes 32 bins: its 32 warps each sum a run of the chunks (coalesced over the
+// bins), the runs' totals are scanned in shared memory, and each warp rewrites
+// its run. One thread per bin walked all chunks alone: five CTAs and 0.27 ms
+// for 1000 chunks x 1250 bins, now 25 us.
+constexpr int kScanRuns = 32;
+__global__ void __launch_bounds__(32 * kScanRuns)
+    k_column_scan(int32_t *__restrict__ m, int n_chunks, int nb, int64_t *__restrict__ totals) {
+    __shared__ int32_t s_run[kScanRuns][32];
+    const int lane = threadIdx.x & 31, run = threadIdx.x >> 5;
+    const int64_t b = int64_t(blockIdx.x) * 32 + lane;
+    const int per = (n_chunks + kScanRuns - 1) / kScanRuns;
+    const int c0 = min(run * per, n_chunks), c1 = min(c0 + per, n_chunks);
+    int32_t own = 0;
+    if (b < nb)
+        for (int c = c0; c < c1; ++c) own += m[int64_t(c) * nb + b];
+    s_run[run][lane] = own;
+    __syncthreads();
+    int32_t at = 0;
+    for (int q = 0; q < run; ++q) at += s_run[q][lane];
     if (b >= nb) return;
-    int32_t run = 0;
-    for (int c = 0; c < n_chunks; ++c) {
-        int64_t k = int64_t(c) * nb + b;
-        int32_t v = m[k];
-        m[k] = run;
-        run += v;
+    for (int c = c0; c < c1; ++c) {
+        const int64_t k = int64_t(c) * nb + b;
+        const int32_t v = m[k];
+        m[k] = at;
+        at += v;
     }
-    totals[b] = run;
+    if (run == kScanRuns - 1) totals[b] = at;
 }
 
 // One warp per chunk: walk the chunk's contributions in pixel order and place
@@ -1296,19 +1297,6 @@ __global__ void k_compact_rows(const int64_t *__restrict__ row_ptr, int64_t n_ro
     }
 }
 
-// normalization::<false> (prepared.rs:229-262) via row() (prepared.rs:1011):
-// n = n + w*x, strictly sequential per row.
-__global__ void k_denominators(const int64_t *__restrict__ row_ptr, int64_t n_rows,
-                               const int32_t *__restrict__ col, const double *__restrict__ w,
-                               const double *__restrict__ norm, double *__restrict__ den) {
-    for (int64_t r = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; r < n_rows;
-         r += int64_t(gridDim.x) * blockDim.x) {
-        double n = 0.0;
-        for (int64_t k = row_ptr[r]; k < row_ptr[r + 1]; ++k) n = n + w[k] * norm[col[k]];
-        den[r] = n;
-    }
-}
-
 unsigned grid_for(int64_t n, int threads = 256) {
     int64_t b = (n + threads - 1) / threads;
     if (b < 1) b = 1;
@@ -1349,7 +1337,7 @@ void transpose(const int32_t *cbin, const double *cw, const int32_t *cpix,
     DG_CUDA(cudaGetLastError());
     DeviceArray<int64_t> totals;
     totals.alloc(size_t(nb) + 1);
-    k_column_scan<<<(nb + 255) / 256, 256, 0, s>>>(m.ptr, n_chunks, nb, totals.ptr);
+    k_column_scan<<<(nb + 31) / 32, 32 * kScanRuns, 0, s>>>(m.ptr, n_chunks, nb, totals.ptr);
     DG_CUDA(cudaGetLastError());
     out.n_rows = nb;
     out.nnz = ncoo;
@@ -1586,7 +1574,7 @@ void build_table_2d(const dg_geometry &geom, const dg_method &m, int32_t dim1, i
             for (int64_t b0 = 0; b0 < ns; b0 += batch) {
                 const int nbat = int(std::min<int64_t>(batch, ns - b0));
                 DG_CUDA(cudaMemsetAsync(hits.ptr, 0, size_t(nbat) * nb * 4, s));
-                k_sample2d<<<nbat, 256, 0, s>>>(gp, g, dim2, sing.ptr + b0, hits.ptr);
+                k_sample2d<<<dim3(unsigned(nbat), kSampleSlices), 256, 0, s>>>(gp, g, dim2, sing.ptr + b0, hits.ptr);
                 k_sample2d_count<<<nbat, 256, 0, s>>>(sing.ptr + b0, nb, hits.ptr, count.ptr);
                 DG_CUDA(cudaGetLastError());
             }
@@ -1599,9 +1587,9 @@ void build_table_2d(const dg_geometry &geom, const dg_method &m, int32_t dim1, i
         for (int64_t b0 = 0; b0 < ns; b0 += batch) {
             const int nbat = int(std::min<int64_t>(batch, ns - b0));
             DG_CUDA(cudaMemsetAsync(hits.ptr, 0, size_t(nbat) * nb * 4, s));
-            k_sample2d<<<nbat, 256, 0, s>>>(gp, g, dim2, sing.ptr + b0, hits.ptr);
-            k_sample2d_fill<<<nbat, 32, 0, s>>>(sing.ptr + b0, nb, hits.ptr, off.ptr, cbin.ptr,
-                                                cw.ptr, cpix.ptr);
+            k_sample2d<<<dim3(unsigned(nbat), kSampleSlices), 256, 0, s>>>(gp, g, dim2, sing.ptr + b0, hits.ptr);
+            k_hits_fill<<<nbat, 32, 0, s>>>(sing.ptr + b0, nb, hits.ptr, off.ptr, cbin.ptr,
+                                            cw.ptr, cpix.ptr);
             DG_CUDA(cudaGetLastError());
         }
     }
@@ -1726,7 +1714,7 @@ void build_table(const dg_geometry &geom, const dg_method &m, int32_t dim1, int3
         out.guard_corners = int64_t(to_host(guard.ptr, 1, s)[0]);
         if (ns > sing_cap) fail(DG_UNSUPPORTED, "too many singular pixels for sampling");
         out.singular_pixels = ns;
-        DeviceArray<int32_t> hits, slot;
+        DeviceArray<int32_t> hits;
         if (ns > 0) {
             // Sort the singular list so slots are deterministic.
             std::vector<int32_t> hs = to_host(sing.ptr, size_t(ns), s);
@@ -1734,21 +1722,18 @@ void build_table(const dg_geometry &geom, const dg_method &m, int32_t dim1, int3
             DG_CUDA(cudaMemcpyAsync(sing.ptr, hs.data(), hs.size() * 4, cudaMemcpyHostToDevice, s));
             hits.alloc(size_t(ns) * nb);
             DG_CUDA(cudaMemsetAsync(hits.ptr, 0, hits.bytes(), s));
-            k_sample<<<ns, 256, 0, s>>>(g, dim2, sing.ptr, nb, mn, a.r1, clamp_low, hits.ptr);
+            k_sample<<<dim3(unsigned(ns), kSampleSlices), 256, 0, s>>>(g, dim2, sing.ptr, nb, mn, a.r1, clamp_low, hits.ptr);
             DG_CUDA(cudaGetLastError());
             k_sample_count<<<ns, 256, 0, s>>>(sing.ptr, nb, hits.ptr, count.ptr);
             DG_CUDA(cudaGetLastError());
-            std::vector<int32_t> hslot(size_t(npix), -1);
-            for (int32_t i = 0; i < ns; ++i) hslot[size_t(hs[size_t(i)])] = i;
-            slot.alloc(size_t(npix));
-            DG_CUDA(cudaMemcpyAsync(slot.ptr, hslot.data(), size_t(npix) * 4,
-                                    cudaMemcpyHostToDevice, s));
-            DG_CUDA(cudaStreamSynchronize(s));
+            DG_CUDA(cudaStreamSynchronize(s));  // hs is read by the copy
         }
         ncoo = scan_counts();
-        k_ps1d_fill<<<grid_for(npix, 128), 128, 0, s>>>(a, off.ptr, ns ? slot.ptr : nullptr,
-                                                        hits.ptr, cbin.ptr, cw.ptr, cpix.ptr,
+        k_ps1d_fill<<<grid_for(npix, 128), 128, 0, s>>>(a, off.ptr, cbin.ptr, cw.ptr, cpix.ptr,
                                                         flags.ptr);
+        if (ns > 0)
+            k_hits_fill<<<ns, 32, 0, s>>>(sing.ptr, nb, hits.ptr, off.ptr, cbin.ptr, cw.ptr,
+                                          cpix.ptr);
         DG_CUDA(cudaGetLastError());
     } else if (m.kind == DG_METHOD_COUNTING) {
         double mn, mx, step;
@@ -1852,32 +1837,29 @@ void build_table(const dg_geometry &geom, const dg_method &m, int32_t dim1, int3
         const int32_t ns = to_host(n_sing.ptr, 1, s)[0];
         if (ns > sing_cap) fail(DG_UNSUPPORTED, "too many singular pixels for sampling");
         out.singular_pixels = ns;
-        DeviceArray<int32_t> hits, slot;
+        DeviceArray<int32_t> hits;
         if (ns > 0) {
             std::vector<int32_t> hs = to_host(sing.ptr, size_t(ns), s);
             std::sort(hs.begin(), hs.end());
             DG_CUDA(cudaMemcpyAsync(sing.ptr, hs.data(), hs.size() * 4, cudaMemcpyHostToDevice, s));
             hits.alloc(size_t(ns) * nb);
             DG_CUDA(cudaMemsetAsync(hits.ptr, 0, hits.bytes(), s));
-            k_sample<<<ns, 256, 0, s>>>(g, dim2, sing.ptr, nb, a.r0, a.r1,
+            k_sample<<<dim3(unsigned(ns), kSampleSlices), 256, 0, s>>>(g, dim2, sing.ptr, nb, a.r0, a.r1,
                                         m.has_radial_range ? 0 : 1, hits.ptr);
             DG_CUDA(cudaGetLastError());
             k_sample_count<<<ns, 256, 0, s>>>(sing.ptr, nb, hits.ptr, count.ptr);
             DG_CUDA(cudaGetLastError());
-            std::vector<int32_t> hslot(size_t(npix), -1);
-            for (int32_t i = 0; i < ns; ++i) hslot[size_t(hs[size_t(i)])] = i;
-            slot.alloc(size_t(npix));
-            DG_CUDA(cudaMemcpyAsync(slot.ptr, hslot.data(), size_t(npix) * 4,
-                                    cudaMemcpyHostToDevice, s));
-            DG_CUDA(cudaStreamSynchronize(s));
+            DG_CUDA(cudaStreamSynchronize(s));  // hs is read by the copy
         }
         ncoo = scan_counts();
         if (ncoo > 64ll * 1024 * 1024)
             fail(DG_UNSUPPORTED, "pyFAI-compatible splitting exceeds the 64-million-entry memory "
                                  "bound; reduce binning.");
-        k_pf1d_fill<<<grid_for(npix, 128), 128, 0, s>>>(a, off.ptr, ns ? slot.ptr : nullptr,
-                                                        hits.ptr, cbin.ptr, cw.ptr, cpix.ptr,
+        k_pf1d_fill<<<grid_for(npix, 128), 128, 0, s>>>(a, off.ptr, cbin.ptr, cw.ptr, cpix.ptr,
                                                         flags.ptr);
+        if (ns > 0)
+            k_hits_fill<<<ns, 32, 0, s>>>(sing.ptr, nb, hits.ptr, off.ptr, cbin.ptr, cw.ptr,
+                                          cpix.ptr);
         DG_CUDA(cudaGetLastError());
     } else {
         fail(DG_UNSUPPORTED, "unknown integration method");
@@ -1941,12 +1923,6 @@ void compact_table(const DeviceCsr &full, const uint8_t *d_mask, int32_t n_pixel
                                                              out.row_ptr.ptr);
     DG_CUDA(cudaGetLastError());
     DG_CUDA(cudaStreamSynchronize(s));
-}
-
-void denominators(const DeviceCsr &t, const double *d_norm, cudaStream_t s, double *d_den) {
-    k_denominators<<<grid_for(t.n_rows, 128), 128, 0, s>>>(t.row_ptr.ptr, t.n_rows, t.col.ptr,
-                                                           t.w.ptr, d_norm, d_den);
-    DG_CUDA(cudaGetLastError());
 }
 
 }  // namespace dg

@@ -2368,19 +2368,49 @@ __global__ void __launch_bounds__(256)
     out_cnt[o] = s_o[3][wr][wf];
 }
 
+// Rows of a table at plan time: T threads walk a row's entries together (32:
+// eight rows per CTA; 256: a CTA per row), coalesced, and add their partial
+// results in a fixed order. One thread per row read 8-byte words from 32 rows
+// at once and left the chip idle (ten CTAs for 1250 rows): k_pack took 4.30 ms
+// and the separate denominator pass 1.46 ms on the Pilatus-1M table (2.5 M
+// entries); now one pass of 36 us for both.
+constexpr int kPackThreads = 256;
+// Rows of more than 256 entries on average take a CTA each; shorter ones (2D
+// bins, about 70 entries) would leave most of its threads without one.
+inline bool pack_cta_per_row(int64_t nnz, int64_t n_rows) { return nnz > 256 * n_rows; }
+
+// Sum over the T threads of a row, in every thread (T = 32) or in thread 0 of
+// the CTA (T = 256). Every thread of the warp (CTA) calls it.
+template <int T>
+__device__ __forceinline__ double row_sum(double v, double *s_red) {
+    v = warp_sum_d(v);
+    if constexpr (T > 32) {
+        if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
+        __syncthreads();
+        v = 0.0;
+        for (int w = 0; w < T / 32; ++w) v = __dadd_rn(v, s_red[w]);
+        __syncthreads();
+    }
+    return v;
+}
+
 // Entries for the per-frame-mask gather, {pixel, w, w*norm} in FP32 (the
-// product formed in FP64), and the strict FP64 weight sum of every row.
-__global__ void k_pack_raw(const int64_t *__restrict__ row_ptr, int n_rows,
-                           const int32_t *__restrict__ col, const double *__restrict__ w,
-                           const double *__restrict__ norm, float4 *__restrict__ entry_raw,
-                           double *__restrict__ cnt, int flip_rows, int flip_cols) {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
+// product formed in FP64), and the FP64 weight sum of every row.
+template <int T>
+__global__ void __launch_bounds__(kPackThreads)
+    k_pack_raw(const int64_t *__restrict__ row_ptr, int n_rows, const int32_t *__restrict__ col,
+               const double *__restrict__ w, const double *__restrict__ norm,
+               float4 *__restrict__ entry_raw, double *__restrict__ cnt, int flip_rows,
+               int flip_cols) {
+    __shared__ double s_red[kPackThreads / 32];
+    const int r = blockIdx.x * (kPackThreads / T) + int(threadIdx.x) / T;
+    const int li = int(threadIdx.x) % T;
     if (r >= n_rows) return;
     double sum = 0.0;
-    for (int64_t k = row_ptr[r]; k < row_ptr[r + 1]; ++k) {
+    for (int64_t k = row_ptr[r] + li; k < row_ptr[r + 1]; k += T) {
         const int32_t j = col[k];
         const double c = w[k];
-        sum += c;
+        sum = __dadd_rn(sum, c);
         // the frame's pixel (rows flipped for InputOrder::FlipVertical)
         int32_t jf = j;
         if (flip_rows) {
@@ -2390,7 +2420,8 @@ __global__ void k_pack_raw(const int64_t *__restrict__ row_ptr, int n_rows,
         entry_raw[k] = make_float4(__int_as_float(jf), __double2float_rn(c),
                                    __double2float_rn(c * norm[j]), 0.f);
     }
-    cnt[r] = sum;
+    sum = row_sum<T>(sum, s_red);
+    if (li == 0) cnt[r] = sum;
 }
 
 // Packs the masked f64 table into the gather's entry formats and computes
@@ -2417,20 +2448,27 @@ __global__ void k_px_norm(const double *__restrict__ norm, int64_t n_px, int row
     }
 }
 
-__global__ void k_pack(const int64_t *__restrict__ row_ptr, int n_rows,
-                       const int32_t *__restrict__ col, const double *__restrict__ w,
-                       const double *__restrict__ norm, int2 *__restrict__ entry,
-                       float4 *__restrict__ entry_std, float *__restrict__ entry_nlo,
-                       double *__restrict__ den_std, int32_t *__restrict__ valid_std,
-                       int32_t *__restrict__ first_valid, int32_t *__restrict__ origin) {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
+template <int T>
+__global__ void __launch_bounds__(kPackThreads)
+    k_pack(const int64_t *__restrict__ row_ptr, int n_rows, const int32_t *__restrict__ col,
+           const double *__restrict__ w, const double *__restrict__ norm,
+           int2 *__restrict__ entry, float4 *__restrict__ entry_std,
+           float *__restrict__ entry_nlo, double *__restrict__ den,
+           double *__restrict__ den_std, int32_t *__restrict__ valid_std,
+           int32_t *__restrict__ first_valid, int32_t *__restrict__ origin) {
+    __shared__ double s_red[kPackThreads / 32];
+    __shared__ double s_heavy[kPackThreads / 32];
+    __shared__ int s_int[3][kPackThreads / 32];
+    const int r = blockIdx.x * (kPackThreads / T) + int(threadIdx.x) / T;
+    const int li = int(threadIdx.x) % T;
     if (r >= n_rows) return;
-    double sw = 0.0, heaviest = 0.0;
-    int valid = 0, first = -1, org = -1;
-    for (int64_t k = row_ptr[r]; k < row_ptr[r + 1]; ++k) {
+    double all = 0.0, sw = 0.0, heaviest = 0.0;
+    int valid = 0, first = INT_MAX, org = INT_MAX;
+    for (int64_t k = row_ptr[r] + li; k < row_ptr[r + 1]; k += T) {
         int32_t j = col[k];
         double c = w[k], n = norm[j];
-        double ww = c * n;
+        double ww = __dmul_rn(c, n);
+        all = __dadd_rn(all, ww);
         bool ok = isfinite(n) && n > 0.0 && isfinite(c) && c > 0.0 && isfinite(ww) && ww > 0.0;
         float cf = __double2float_rn(c);
         entry[k] = make_int2(j, __float_as_int(cf));
@@ -2439,38 +2477,72 @@ __global__ void k_pack(const int64_t *__restrict__ row_ptr, int n_rows,
                                    ok ? __double2float_rn(c / n) : 0.f);
         entry_nlo[k] = ok ? __double2float_rn(n - double(nf)) : 0.f;
         if (ok) {
-            sw += ww;
+            sw = __dadd_rn(sw, ww);
             ++valid;
-            if (first < 0) first = int(k);
+            first = min(first, int(k));
             if (ww > heaviest) {  // the first of equally heavy entries
                 heaviest = ww;
                 org = int(k);
             }
         }
     }
+    all = row_sum<T>(all, s_red);
+    sw = row_sum<T>(sw, s_red);
+    auto heavier = [&](double h, int o) {
+        if (h > heaviest || (h == heaviest && o < org)) {
+            heaviest = h;
+            org = o;
+        }
+    };
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) {
+        valid += __shfl_xor_sync(0xffffffffu, valid, m);
+        first = min(first, __shfl_xor_sync(0xffffffffu, first, m));
+        const double h = __shfl_xor_sync(0xffffffffu, heaviest, m);
+        heavier(h, __shfl_xor_sync(0xffffffffu, org, m));
+    }
+    if constexpr (T > 32) {
+        const int warp = int(threadIdx.x) >> 5;
+        if ((threadIdx.x & 31) == 0) {
+            s_heavy[warp] = heaviest;
+            s_int[0][warp] = org;
+            s_int[1][warp] = valid;
+            s_int[2][warp] = first;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int q = 1; q < T / 32; ++q) {
+                heavier(s_heavy[q], s_int[0][q]);
+                valid += s_int[1][q];
+                first = min(first, s_int[2][q]);
+            }
+    }
+    if (li != 0) return;
+    den[r] = all;
     den_std[r] = sw;
     valid_std[r] = valid;
-    first_valid[r] = first;
-    origin[r] = org;
+    first_valid[r] = valid ? first : -1;
+    origin[r] = valid ? org : -1;
 }
 
 // bounds[r * (n_strips + 1) + s]: first entry of row r whose pixel lies in
-// strip s or later (columns within a row are ascending).
+// strip s or later (columns within a row are ascending). A thread per (row,
+// strip): the searches of one row by one thread ran one after another
+// (0.30 ms for 1250 rows x 67 strips).
 __global__ void k_strip_bounds(const int64_t *__restrict__ row_ptr, int n_rows,
                                const int32_t *__restrict__ col, int n_strips, int64_t strip_px,
                                int32_t *__restrict__ bounds) {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n_rows) return;
-    int64_t b = row_ptr[r], e = row_ptr[r + 1];
-    int32_t *out = bounds + int64_t(r) * (n_strips + 1);
-    for (int s = 0; s <= n_strips; ++s) {
-        int64_t key = int64_t(s) * strip_px, lo = b, hi = e;
+    const int64_t n = int64_t(n_rows) * (n_strips + 1);
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n;
+         i += int64_t(gridDim.x) * blockDim.x) {
+        const int64_t r = i / (n_strips + 1), st = i - r * (n_strips + 1);
+        int64_t key = st * strip_px, lo = row_ptr[r], hi = row_ptr[r + 1];
         while (lo < hi) {
             int64_t mid = (lo + hi) >> 1;
             if (int64_t(col[mid]) < key) lo = mid + 1;
             else hi = mid;
         }
-        out[s] = int32_t(lo);
+        bounds[i] = int32_t(lo);
     }
 }
 
@@ -2664,17 +2736,39 @@ void gather_kernel_time(GatherTable &t, bool reset, double *ms, int64_t *gather_
     }
 }
 
+namespace {
+// Runs of consecutive segments of one strip, at most max_segs segments and
+// `cap` entries each: emit(first segment, segments).
+template <class Emit>
+void group_segments(const std::vector<int4> &segs, const std::vector<int32_t> &strip_first, int cap,
+                    int max_segs, Emit &&emit) {
+    for (size_t st = 0; st + 1 < strip_first.size(); ++st) {
+        int first = strip_first[st], entries = 0;
+        for (int i = first; i < strip_first[st + 1]; ++i) {
+            const int len = segs[size_t(i)].z - segs[size_t(i)].y;
+            if (i - first == max_segs || entries + len > cap) {
+                emit(first, i - first);
+                first = i;
+                entries = 0;
+            }
+            entries += len;
+        }
+        if (strip_first[st + 1] > first) emit(first, strip_first[st + 1] - first);
+    }
+}
+
+__global__ void k_flip_rows(int2 *__restrict__ entry, float4 *__restrict__ entry_std, int64_t nnz,
+                            int32_t *__restrict__ px, int64_t n_px, int rows, int cols);
+}  // namespace
+
 // Frame-lane units (k_gather_fl): runs of at most kFlSegs segments and
 // kFlECap entries of one strip, split in halves by entries until each holds
 // at most kFlDCap distinct pixels; then their pixel lists and entry pairs.
-template <class Group>
 void build_fl_units(GatherTable &out, const DeviceCsr &table, const std::vector<int4> &segs,
-                    Group &&group, cudaStream_t s) {
+                    std::vector<int4> fl, cudaStream_t s) {
     out.fl_n_units = 0;
     out.fl_pair_as = nullptr;
     if (segs.empty() || table.nnz > INT32_MAX) return;
-    std::vector<int4> fl;
-    group(kFlECap, kFlSegs, fl);
     DeviceArray<int4> d_units;
     DeviceArray<int32_t> d_count;
     std::vector<int32_t> count;
@@ -3068,18 +3162,22 @@ void make_gather_table(const DeviceCsr &table, const double *d_norm, int32_t dim
     out.valid_std.alloc(size_t(table.n_rows));
     out.first_valid.alloc(size_t(table.n_rows));
     out.origin.alloc(size_t(table.n_rows));
-    denominators(table, d_norm, s, out.den.ptr);
     const int64_t n_px = int64_t(dim1) * dim2;
     out.px_norm.alloc(size_t(std::max<int64_t>(n_px, 1)));
     if (n_px > 0)
         k_px_norm<<<unsigned(std::min<int64_t>((n_px + 255) / 256, 148 * 16)), 256, 0, s>>>(
             d_norm, n_px, 0, 0, out.px_norm.ptr);
-    const unsigned rb = unsigned((table.n_rows + 127) / 128);
-    if (table.n_rows > 0)
-        k_pack<<<rb, 128, 0, s>>>(table.row_ptr.ptr, int(table.n_rows), table.col.ptr, table.w.ptr,
-                                  d_norm, out.entry.ptr, out.entry_std.ptr, out.entry_nlo.ptr,
-                                  out.den_std.ptr, out.valid_std.ptr, out.first_valid.ptr,
-                                  out.origin.ptr);
+    if (table.n_rows > 0) {
+#define DG_PACK_ARGS                                                                          \
+    table.row_ptr.ptr, int(table.n_rows), table.col.ptr, table.w.ptr, d_norm, out.entry.ptr,  \
+        out.entry_std.ptr, out.entry_nlo.ptr, out.den.ptr, out.den_std.ptr, out.valid_std.ptr, \
+        out.first_valid.ptr, out.origin.ptr
+        if (pack_cta_per_row(table.nnz, table.n_rows))
+            k_pack<256><<<unsigned(table.n_rows), kPackThreads, 0, s>>>(DG_PACK_ARGS);
+        else
+            k_pack<32><<<unsigned((table.n_rows + 7) / 8), kPackThreads, 0, s>>>(DG_PACK_ARGS);
+#undef DG_PACK_ARGS
+    }
     DG_CUDA(cudaGetLastError());
 
     // Segments: (row, strip) runs from per-row strip bounds found on the
@@ -3089,8 +3187,9 @@ void make_gather_table(const DeviceCsr &table, const double *d_norm, int32_t dim
     DeviceArray<int32_t> bounds;
     bounds.alloc(size_t(nb * (n_strips + 1)));
     if (nb > 0)
-        k_strip_bounds<<<rb, 128, 0, s>>>(table.row_ptr.ptr, int(nb), table.col.ptr, n_strips,
-                                          int64_t(strip_rows) * dim2, bounds.ptr);
+        k_strip_bounds<<<unsigned(std::min<int64_t>((nb * (n_strips + 1) + 255) / 256, 148 * 64)), 256,
+                         0, s>>>(table.row_ptr.ptr, int(nb), table.col.ptr, n_strips,
+                                 int64_t(strip_rows) * dim2, bounds.ptr);
     DG_CUDA(cudaGetLastError());
     std::vector<int32_t> hb(size_t(nb * (n_strips + 1)));
     std::vector<int64_t> rp(size_t(nb) + 1);
@@ -3115,24 +3214,8 @@ void make_gather_table(const DeviceCsr &table, const double *d_norm, int32_t dim
         }
     }
     strip_first[size_t(n_strips)] = int32_t(segs.size());
-    // Units: runs of consecutive segments of one strip, at most max_segs
-    // segments and `cap` entries each.
-    auto group = [&](int cap, int max_segs, auto &&emit) {
-        for (int st = 0; st < n_strips; ++st) {
-            int first = strip_first[size_t(st)], entries = 0;
-            for (int i = first; i < strip_first[size_t(st) + 1]; ++i) {
-                const int len = segs[size_t(i)].z - segs[size_t(i)].y;
-                if (i - first == max_segs || entries + len > cap) {
-                    emit(first, i - first);
-                    first = i;
-                    entries = 0;
-                }
-                entries += len;
-            }
-            if (strip_first[size_t(st) + 1] > first) emit(first, strip_first[size_t(st) + 1] - first);
-        }
-    };
-    group(kUnitCap, kWarps, [&](int first, int n) { units.push_back(make_int2(first, n)); });
+    group_segments(segs, strip_first, kUnitCap, kWarps,
+                   [&](int first, int n) { units.push_back(make_int2(first, n)); });
     // Row -> its segments, in strip order (the finalize's fixed fold order).
     std::vector<int32_t> row_seg(size_t(nb) + 1, 0), seg_ids(segs.size());
     for (int64_t r = 0; r < nb; ++r) row_seg[size_t(r) + 1] = row_seg[size_t(r)] + seg_count[size_t(r)];
@@ -3194,9 +3277,32 @@ void make_gather_table(const DeviceCsr &table, const double *d_norm, int32_t dim
         out.rw_n_items = int32_t(rw_items.size());
     }
     DG_CUDA(cudaStreamSynchronize(s));
-    build_fl_units(out, table, segs, [&](int cap, int max_segs, std::vector<int4> &fl) {
-        group(cap, max_segs, [&](int first, int n) { fl.push_back(make_int4(first, n, 0, 0)); });
-    }, s);
+    out.strip_first = std::move(strip_first);
+}
+
+// Frame-lane units are built when mapping 5 or 6 is selected or timed, as the
+// bin tiles are: a plan that runs neither (the default mapping, row warps, bin
+// tiles) does not pay for them. Their build took 1.5 ms of device time, four
+// launches with a host round trip each, of a Pilatus-1M plan's creation.
+void ensure_fl_units(GatherTable &t, const DeviceCsr &table, cudaStream_t s) {
+    if (t.fl_built) return;
+    std::vector<int4> segs(static_cast<size_t>(t.n_segments));
+    if (!segs.empty()) {
+        DG_CUDA(cudaMemcpyAsync(segs.data(), t.seg.ptr, segs.size() * sizeof(int4),
+                                cudaMemcpyDeviceToHost, s));
+        DG_CUDA(cudaStreamSynchronize(s));
+    }
+    std::vector<int4> fl;
+    group_segments(segs, t.strip_first, kFlECap, kFlSegs,
+                   [&](int first, int n) { fl.push_back(make_int4(first, n, 0, 0)); });
+    build_fl_units(t, table, segs, std::move(fl), s);
+    if (t.flip_rows && t.fl_px.ptr) {  // as flip_gather_rows did for the entries
+        k_flip_rows<<<148 * 8, 256, 0, s>>>(nullptr, nullptr, 0, t.fl_px.ptr,
+                                            int64_t(t.fl_px.count), t.flip_rows, t.flip_cols);
+        DG_CUDA(cudaGetLastError());
+        DG_CUDA(cudaStreamSynchronize(s));
+    }
+    t.fl_built = true;
 }
 
 bool gather_writes_results(const GatherTable &t) {
@@ -3457,22 +3563,27 @@ void flip_gather_rows(GatherTable &t, int32_t dim1, int32_t dim2, cudaStream_t s
     if (t.px_norm.ptr && half > 0)
         k_flip_px_norm<<<unsigned(std::min<int64_t>((half + 255) / 256, 148 * 16)), 256, 0, s>>>(
             t.px_norm.ptr, dim1, dim2);
-    const int64_t n_px = t.fl_px.ptr ? int64_t(t.fl_px.count) : 0;
-    if (t.nnz + n_px > 0)
-        k_flip_rows<<<148 * 8, 256, 0, s>>>(t.entry.ptr, t.entry_std.ptr, t.nnz, t.fl_px.ptr,
-                                            n_px, dim1, dim2);
+    if (t.nnz > 0)
+        k_flip_rows<<<148 * 8, 256, 0, s>>>(t.entry.ptr, t.entry_std.ptr, t.nnz, nullptr, 0, dim1,
+                                            dim2);
     DG_CUDA(cudaGetLastError());
-    // bin tiles are built later (ensure_bin_tiles) and flipped then
+    // bin tiles and frame-lane units are built later and flipped then
 }
 
 void prepare_raw(GatherTable &t, const DeviceCsr &table, const double *d_norm, cudaStream_t s) {
     if (t.cnt.ptr) return;
     t.entry_raw.alloc(std::max<size_t>(size_t(table.nnz), 1));
     t.cnt.alloc(std::max<size_t>(size_t(table.n_rows), 1));
-    if (table.n_rows > 0)
-        k_pack_raw<<<unsigned((table.n_rows + 127) / 128), 128, 0, s>>>(
-            table.row_ptr.ptr, int(table.n_rows), table.col.ptr, table.w.ptr, d_norm,
-            t.entry_raw.ptr, t.cnt.ptr, t.flip_rows, t.flip_cols);
+    if (table.n_rows > 0) {
+#define DG_PACK_ARGS                                                                     \
+    table.row_ptr.ptr, int(table.n_rows), table.col.ptr, table.w.ptr, d_norm,            \
+        t.entry_raw.ptr, t.cnt.ptr, t.flip_rows, t.flip_cols
+        if (pack_cta_per_row(table.nnz, table.n_rows))
+            k_pack_raw<256><<<unsigned(table.n_rows), kPackThreads, 0, s>>>(DG_PACK_ARGS);
+        else
+            k_pack_raw<32><<<unsigned((table.n_rows + 7) / 8), kPackThreads, 0, s>>>(DG_PACK_ARGS);
+#undef DG_PACK_ARGS
+    }
     DG_CUDA(cudaGetLastError());
 }
 

@@ -152,11 +152,9 @@ struct BuildResult {
 void build_table(const dg_geometry &g, const dg_method &m, int32_t dim1, int32_t dim2,
                  int32_t n_radial, int32_t n_azimuthal, const double *azimuthal_range,
                  cudaStream_t stream, BuildResult &out);
-// Order-preserving mask compaction (fixed_table) + strict f64 denominators.
+// Order-preserving mask compaction (fixed_table).
 void compact_table(const DeviceCsr &full, const uint8_t *d_mask, int32_t n_pixels,
                    cudaStream_t stream, DeviceCsr &out);
-void denominators(const DeviceCsr &table, const double *d_norm, cudaStream_t stream,
-                  double *d_den);
 // Device FP64 primitives on arrays: 0 correctly rounded atan2(a, b), 1 its
 // sin(a), 2 CUDA atan2, 3 CUDA sin.
 void eval_math(int which, const double *a, const double *b, int64_t n, double *out,
@@ -288,6 +286,8 @@ struct GatherTable {
     // Frame-lane layout (k_gather_fl): units of segments with a bounded
     // number of distinct pixels, their pixel lists (a fixed stride apart) and
     // the entries in unit order as pairs, columns as indices into the lists.
+    bool fl_built = false;            // ensure_fl_units has run
+    std::vector<int32_t> strip_first; // first segment of every strip, then n_segments
     int32_t fl_n_units = 0;
     DeviceArray<int4> fl_unit;        // {first segment, segment count, first pair, pixels}
     DeviceArray<int32_t> fl_px;
@@ -410,6 +410,8 @@ void flip_gather_rows(GatherTable &t, int32_t dim1, int32_t dim2, cudaStream_t s
 // table on first use (the autotuner, or selecting the mapping); idempotent.
 void ensure_bin_tiles(GatherTable &t, const DeviceCsr &table, int variant, cudaStream_t s);
 bool gather_variant_needs_tiles(int variant);
+// Frame-lane units of mappings 5 and 6, built on first use; idempotent.
+void ensure_fl_units(GatherTable &t, const DeviceCsr &table, cudaStream_t s);
 // Throws DG_TIMEOUT (once) when a bin-tile launch of this table gave up a
 // pipeline wait; bin_tile_wait_failed only reports and clears it.
 bool bin_tile_wait_failed(const GatherTable &t);
