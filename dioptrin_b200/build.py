@@ -27,6 +27,7 @@ COMMON = ["-std=c++17", "-O3", "-lineinfo", "--expt-relaxed-constexpr",
           "-Xcompiler", "-fPIC,-ffp-contract=off,-fvisibility=hidden",
           "-I", os.path.join(ROOT, "include")]
 SOURCES = {
+    "dg_alloc.cu": [],
     "dg_build.cu": ["-fmad=false"],
     "dg_scan.cu": [],
     "dg_gather.cu": [],

@@ -230,6 +230,8 @@ dg_status dg_plan_create(const dg_geometry *geometry, const dg_method *method,
         DG_CUDA(cudaEventCreate(&e0));
         DG_CUDA(cudaEventCreate(&e1));
         DG_CUDA(cudaEventRecord(e0, s));
+        // The build's arrays are used on s alone until it is synchronised below.
+        dg::AllocScope alloc(s);
         dg::BuildResult built;
         try {
             dg::build_table(*geometry, *method, dim1, dim2, n_radial, n_azimuthal,
@@ -294,7 +296,10 @@ dg_status dg_plan_destroy(dg_plan *plan) {
             int prev = -1;
             cudaGetDevice(&prev);
             cudaSetDevice(plan->device);
-            if (plan->stream) cudaStreamSynchronize(plan->stream);
+            // Callers' streams may still run on the tables: wait for them once,
+            // then every array is freed without waiting.
+            (void)cudaDeviceSynchronize();
+            dg::AllocScope alloc(dg::idle_stream());
             plan->full = dg::DeviceCsr();
             plan->table = dg::DeviceCsr();
             plan->norm.release();

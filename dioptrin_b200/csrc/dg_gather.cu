@@ -3118,6 +3118,7 @@ void ensure_bin_tiles(GatherTable &t, const DeviceCsr &table, int variant, cudaS
     if (variant != 7 && variant != 8) return;
     BinTiles &bt = t.bt[variant - 7];
     if (bt.built) return;
+    AllocScope alloc(s);  // s is synchronised before this returns
     int words = 0, head = 0;
     if (variant == 7) {
         build_bin_tiles<Bt7>(t, bt, table, s);
@@ -3286,6 +3287,7 @@ void make_gather_table(const DeviceCsr &table, const double *d_norm, int32_t dim
 // launches with a host round trip each, of a Pilatus-1M plan's creation.
 void ensure_fl_units(GatherTable &t, const DeviceCsr &table, cudaStream_t s) {
     if (t.fl_built) return;
+    AllocScope alloc(s);  // s is synchronised before this returns
     std::vector<int4> segs(static_cast<size_t>(t.n_segments));
     if (!segs.empty()) {
         DG_CUDA(cudaMemcpyAsync(segs.data(), t.seg.ptr, segs.size() * sizeof(int4),

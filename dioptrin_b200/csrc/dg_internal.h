@@ -25,15 +25,34 @@ void set_last_error(const std::string &message);
 void check_cuda(cudaError_t err, const char *what);
 #define DG_CUDA(call) ::dg::check_cuda((call), #call)
 
+// Device memory from the library's pool (dg_alloc.cu). While an AllocScope
+// lives on a thread, the thread's allocations and frees are ordered on its
+// stream; outside one, an allocation is complete on return and a free waits for
+// the device first.
+void *device_alloc(size_t bytes, int *device);
+void device_free(void *ptr, int device) noexcept;
+struct AllocScope {
+    cudaStream_t stream;
+    const void *outer;
+    explicit AllocScope(cudaStream_t s);
+    ~AllocScope();
+    AllocScope(const AllocScope &) = delete;
+    AllocScope &operator=(const AllocScope &) = delete;
+};
+// The current device's stream for an AllocScope that frees arrays after the
+// device has been synchronised.
+cudaStream_t idle_stream();
+
 // Device allocation owned by a plan; freed with the plan.
 template <typename T>
 struct DeviceArray {
     T *ptr = nullptr;
     size_t count = 0;
+    int device = 0;
     DeviceArray() = default;
     DeviceArray(const DeviceArray &) = delete;
     DeviceArray &operator=(const DeviceArray &) = delete;
-    DeviceArray(DeviceArray &&o) noexcept : ptr(o.ptr), count(o.count) {
+    DeviceArray(DeviceArray &&o) noexcept : ptr(o.ptr), count(o.count), device(o.device) {
         o.ptr = nullptr;
         o.count = 0;
     }
@@ -42,6 +61,7 @@ struct DeviceArray {
             release();
             ptr = o.ptr;
             count = o.count;
+            device = o.device;
             o.ptr = nullptr;
             o.count = 0;
         }
@@ -51,17 +71,11 @@ struct DeviceArray {
     void alloc(size_t n) {
         release();
         if (n == 0) n = 1;
-        cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&ptr), n * sizeof(T));
-        if (e != cudaSuccess) {
-            ptr = nullptr;
-            (void)cudaGetLastError();
-            fail(DG_DEVICE, "device allocation of " + std::to_string(n * sizeof(T)) +
-                                " bytes failed: " + cudaGetErrorString(e));
-        }
+        ptr = static_cast<T *>(device_alloc(n * sizeof(T), &device));
         count = n;
     }
     void release() {
-        if (ptr) cudaFree(ptr);
+        if (ptr) device_free(ptr, device);
         ptr = nullptr;
         count = 0;
     }
