@@ -8,6 +8,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <new>
 
@@ -143,6 +144,21 @@ void check_device(int32_t device) {
     if (device < 0 || device >= count)
         dg::fail(DG_UNAVAILABLE, "CUDA device " + std::to_string(device) + " does not exist (" +
                                      std::to_string(count) + " visible)");
+}
+
+// A device's properties, queried once: cudaGetDeviceProperties takes about 3 ms
+// on a B200, and a Python plan asks for the device's name when it is created.
+const cudaDeviceProp &device_properties(int32_t device) {
+    static std::mutex mu;
+    static auto *const known = new std::map<int32_t, cudaDeviceProp>;
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = known->find(device);
+    if (it == known->end()) {
+        cudaDeviceProp p{};
+        DG_CUDA(cudaGetDeviceProperties(&p, device));
+        it = known->emplace(device, p).first;
+    }
+    return it->second;
 }
 
 void check_frames(const dg_plan *plan, const void *frames, int32_t dtype, int64_t n_frames,
@@ -899,8 +915,7 @@ dg_status dg_device_info_get(int32_t device, dg_device_info *out) {
         std::memset(out, 0, sizeof *out);
         out->device = device;
         check_device(device);
-        cudaDeviceProp p{};
-        DG_CUDA(cudaGetDeviceProperties(&p, device));
+        const cudaDeviceProp &p = device_properties(device);
         out->available = 1;
         out->cc_major = p.major;
         out->cc_minor = p.minor;
