@@ -31,6 +31,7 @@ SOURCES = {
     "dg_build.cu": ["-fmad=false"],
     "dg_scan.cu": [],
     "dg_gather.cu": [],
+    "dg_bins.cu": [],
     "dg_api.cu": [],
     "dg_server.cu": [],
     "dg_bslz4.cu": [],

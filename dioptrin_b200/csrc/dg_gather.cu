@@ -56,7 +56,7 @@
 #include <memory>
 #include <thread>
 
-#include "dg_internal.h"
+#include "dg_gather_common.cuh"
 
 namespace dg {
 namespace {
@@ -76,41 +76,6 @@ constexpr int kFlush = 16;  // terms per lane between double-word folds
 constexpr int kVariantCount = 11;
 constexpr int kSegMax = 256;
 constexpr int kUnitCap = 3008;  // 16-byte entries in the 48 KB default shared memory
-
-// kRaw: the per-frame-mask gather (entries {pixel, w, w*norm}); it sums
-// S = sum w*s, V = sum w^2*max(s,0), N = sum w*norm and C = sum w over the
-// entries whose pixel the frame's mask leaves unmasked.
-enum Mode { kIntensity = 0, kErrors = 1, kSpread = 2, kRaw = 3 };
-
-template <typename P>
-constexpr bool is_float_px() {
-    return std::is_same<P, float>::value || std::is_same<P, double>::value;
-}
-
-// Accumulators per (segment, frame): S = sum c*s, then V = sum c^2*max(s,0),
-// then for the spread B = sum (c/n)*t^2 and A = sum c*t, then for float
-// pixels the weight c*n and the count of non-finite pixels.
-template <int MODE, typename P>
-struct NAcc {
-    static constexpr int value = MODE == kIntensity ? 1
-                                 : MODE == kErrors  ? 2
-                                 : MODE == kRaw     ? 4
-                                                    : (is_float_px<P>() ? 6 : 4);
-};
-constexpr int kSpreadA = 3;  // index of A among the spread's accumulators
-constexpr int kMaxAcc = 6;   // accumulators per (segment, frame), at most
-static_assert(NAcc<kSpread, float>::value <= kMaxAcc && NAcc<kRaw, float>::value <= kMaxAcc,
-              "partial sums are sized for kMaxAcc accumulators");
-
-// Accumulators per frame of a mode, for sizing partial sums at run time.
-inline int n_accumulators(int mode, bool float_px) {
-    return mode == kIntensity ? 1 : mode == kErrors ? 2 : mode == kRaw ? 4 : (float_px ? 6 : 4);
-}
-
-template <typename P>
-constexpr bool is_unsigned_px() {
-    return std::is_same<P, uint16_t>::value || std::is_same<P, uint32_t>::value;
-}
 
 // Double-word FP32 accumulator with a plain FP32 block in front.
 struct AccDW {
@@ -141,42 +106,6 @@ struct AccDW {
         lo = __fsub_rn(t, __fsub_rn(hi, s));
     }
 };
-
-template <typename P>
-__device__ __forceinline__ float load_px(const P *__restrict__ f, uint32_t i) {
-    return float(__ldg(f + i));
-}
-template <>
-__device__ __forceinline__ float load_px<double>(const double *__restrict__ f, uint32_t i) {
-    return __double2float_rn(__ldg(f + i));
-}
-
-// Origin o = s/n of the spread's shift in this frame. The reference shifts
-// by the row's first valid entry (azimuthal.rs:80-82); the spread does not
-// depend on the shift, only its rounding does: the moments lose to
-// cancellation about (mean - o)^2 / variance, so this build shifts by the
-// row's heaviest valid entry (largest c*n, chosen at plan time), which sits
-// at the mean of a bin dominated by one pixel. A float pixel that is not
-// finite there hands the origin to the row's first valid finite entry
-// (entries that are statically invalid carry c = 0).
-template <typename P>
-__device__ __forceinline__ float row_origin(const float4 *__restrict__ entry_std, int origin,
-                                            int first, int row_end,
-                                            const P *__restrict__ frame) {
-    if (origin < 0) return 0.f;
-    float4 e = entry_std[origin];
-    float s = load_px<P>(frame, uint32_t(__float_as_int(e.x)));
-    if (is_float_px<P>() && !isfinite(s)) {
-        for (int k = first; k < row_end; ++k) {
-            const float4 ek = entry_std[k];
-            if (!(ek.y > 0.f)) continue;
-            e = ek;
-            s = load_px<P>(frame, uint32_t(__float_as_int(e.x)));
-            if (isfinite(s)) break;
-        }
-    }
-    return __fdiv_rn(s, e.z);
-}
 
 // Reduce-scatter of V values (a power of two, <= 32) across the 32 lanes of
 // a warp by a fixed butterfly: after the call, lanes 2i and 2i+1 (V = 16),
@@ -816,88 +745,6 @@ static_assert(kFlECap + kFlSegs <= kFlSortMax, "frame-lane units must fit the pl
 static_assert(kFlSegs <= 32, "the unit set-up scans segment lengths in one warp");
 static_assert(kSegMax <= kFlDCap, "a single segment must fit a frame-lane unit");
 
-template <typename P>
-using StagedPx = typename std::conditional<sizeof(P) == 4, P, float>::type;
-
-__device__ __forceinline__ void cp_async4(void *dst, const void *src) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-// The same with the shared-memory address as a 32-bit integer, and a 32-bit
-// shared-memory load: address arithmetic stays in 32 bits.
-__device__ __forceinline__ void cp_async4_s(unsigned d, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-// L2 eviction priority of the bin tiles' 4-byte pixel copies: 0 the default
-// policy, 1 evict-first (frame sectors stream through L2 and leave it to the
-// entry-pair records that a tile's frame groups share), 2 evict-last.
-#ifndef DG_BT_L2HINT
-#define DG_BT_L2HINT 0
-#endif
-__device__ __forceinline__ uint64_t bt_l2_policy() {
-    uint64_t p = 0;
-    if constexpr (DG_BT_L2HINT == 1)
-        asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(p));
-    else if constexpr (DG_BT_L2HINT == 2)
-        asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;\n" : "=l"(p));
-    return p;
-}
-__device__ __forceinline__ void cp_async4_sp(unsigned d, const void *src, uint64_t policy) {
-    if constexpr (DG_BT_L2HINT == 0) {
-        cp_async4_s(d, src);
-    } else {
-        asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], 4, %2;\n" ::"r"(d),
-                     "l"(src), "l"(policy)
-                     : "memory");
-    }
-}
-__device__ __forceinline__ uint32_t lds32(unsigned a) {
-    uint32_t v;
-    asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(v) : "r"(a));
-    return v;
-}
-// A staged 4-byte pixel from its bits.
-template <typename S>
-__device__ __forceinline__ float staged_value(uint32_t b) {
-    if constexpr (std::is_same<S, float>::value) return __uint_as_float(b);
-    else if constexpr (std::is_same<S, int32_t>::value) return float(int32_t(b));
-    else return float(b);
-}
-
-// Packed FP32x2 arithmetic (round to nearest, per element as the scalar
-// operations).
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 pk(float a, float b) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 upk(f2 v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ f2 add2(f2 a, f2 b) {
-    f2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
-    f2 d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-    f2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
 // Two double-word FP32 accumulators (even and odd entries) with a plain
 // FP32 block in front; the fold is AccDW::flush on each half.
 struct Acc2 {
@@ -916,23 +763,6 @@ struct Acc2 {
         const float2 h = upk(hi), l = upk(lo);
         return __dadd_rn(double(h.x) + double(l.x), double(h.y) + double(l.y));
     }
-};
-
-// The same packed partial folded into one FP64 sum instead (both halves
-// added in FP64, even then odd): four registers instead of six.
-struct AccP64 {
-    f2 p;
-    double d;
-    __device__ __forceinline__ void zero() {
-        p = 0ull;
-        d = 0.0;
-    }
-    __device__ __forceinline__ void flush() {
-        const float2 h = upk(p);
-        d = __dadd_rn(__dadd_rn(d, double(h.x)), double(h.y));
-        p = 0ull;
-    }
-    __device__ __forceinline__ double value() const { return d; }
 };
 
 
@@ -1385,861 +1215,6 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// ---------------------------------------------------------------------------
-// Bin-tile gathers (mappings 7 and 8). A tile is ROWS consecutive rows
-// (bins) of the table and 32 * F2 frames (lane = frame; F2 frames per lane,
-// 32 apart). The tile's entries, merged over its rows in pixel order, are cut
-// into chunks of at most DCap distinct pixels and PCap entry pairs; a row's
-// entries inside a chunk are a contiguous run of its CSR row. The CTA walks
-// the tile's chunks in order through a ring of buffers: while chunk k is
-// summed, the next chunk's pixels (4-byte cp.async into frame rows Stride
-// words apart, every warp staging an equal share) and entry pairs (16-byte
-// cp.async) are in flight. There is no CTA-wide barrier per chunk: each
-// buffer has mbarriers for "landed" (every thread's copies) and "summed"
-// (every warp), so a warp whose row has many entries in one chunk can finish
-// it while the others start the next one; a row's load evens out over the
-// tile (rows of a tile hold nearly equal entry counts; their shares of one
-// chunk do not). Every wait is bounded (kBtWaitNs); a warp that gives up
-// ends the tile and sets a flag in mapped host memory that the host reports
-// as DG_TIMEOUT. Warp w owns row w of the tile and keeps its sums in
-// registers for the whole tile (double-word FP32, folded every kBtFoldPairs
-// pairs of the row), then normalises and writes the results itself: no
-// partial sums, no finalize launch. Every row is summed in the same order for
-// every frame and batch.
-// With two frames per lane (mapping 8) every entry pair read from shared
-// memory serves 64 frames: half the broadcast reads per frame, at half the
-// chunk size.
-// The same kernel writes raw sums instead (flag `raw`: S and V, with the
-// row's strict N and C), and in mode kRaw applies per-frame masks on mapping
-// 8's tiles (BtR: two frames per lane, one for 2-byte pixels): a chunk's mask
-// bytes are staged
-// next to its pixels, and a masked entry adds nothing to S, V, N or C. Bytes
-// the kernel loads rather than copies (masks, 2-byte pixels) are loaded with
-// a chunk's copies and stored after the warp has summed the chunk before it.
-
-// One bin-tile layout: rows per tile (= warps per CTA: warp w owns row w),
-// chunk capacities, frames per lane, pairs per unrolled step and the chunk
-// pipeline: BUFS pixel/pair buffers, pixels staged AHEAD chunks before they
-// are summed and records MAHEAD chunks before their pixels. Per-chunk
-// record, fixed size: {pixels D, pairs, first pair, 0}, the rows' pair
-// offsets (ROWS + 1, padded to a multiple of 4 words), then D pixel indices.
-template <int ROWS, int DCAP, int PCAP, int F2, int U2, int BUFS = 3, int AHEAD = 1,
-          int MAHEAD = 1>
-struct BtCfg {
-    static constexpr int kRows = ROWS;
-    static constexpr int kThreads = ROWS * 32;
-    static constexpr int kU2 = U2;
-    static constexpr int kBufs = BUFS;
-    static constexpr int kAhead = AHEAD;
-    static constexpr int kMetaAhead = MAHEAD;
-    // A record slot is rewritten only after every warp has summed the chunk
-    // it held (the buffer waits guarantee that for BUFS + MAHEAD slots).
-    static constexpr int kMetaBufs = BUFS + MAHEAD;
-    // How many chunks a warp may fall behind the fastest one.
-    static constexpr int kLag = AHEAD < MAHEAD ? (AHEAD < BUFS - AHEAD - 1 ? AHEAD : BUFS - AHEAD - 1)
-                                               : (MAHEAD < BUFS - AHEAD - 1 ? MAHEAD : BUFS - AHEAD - 1);
-    static_assert(AHEAD >= 1 && MAHEAD >= 1 && kLag >= 0, "pipeline depths");
-    static_assert(ROWS <= 32, "tile rows are packed in 5 bits at plan time");
-    static constexpr int kDCap = DCAP;          // distinct pixels per chunk
-    static constexpr int kStride = DCAP + 1;    // odd frame-row stride; column DCAP stays 0
-    static constexpr int kPCap = PCAP;          // entry pairs per chunk
-    static constexpr int kF2 = F2;              // frames per lane
-    static constexpr int kFrames = 32 * F2;     // frames per CTA
-    static constexpr int kMetaHead = (4 + ROWS + 1 + 3) / 4 * 4;
-    static constexpr int kMetaWords = kMetaHead + DCAP;
-    // Staging shares: the chunk's pixels are cut into kSlices slices and warp
-    // w stages slice w % kSlices of kStageFrames frames (w / kSlices + j *
-    // ROWS / kSlices), so every warp issues the same number of copies and
-    // reads each pixel index once for all its frames.
-    static constexpr int kSlices = ROWS % 3 == 0 ? 3 : 1;
-    static constexpr int kStageFrames = kFrames * kSlices / ROWS;
-    static_assert(ROWS % kSlices == 0 && (kFrames * kSlices) % ROWS == 0,
-                  "staging shares must divide evenly");
-    static_assert(kMetaWords % 4 == 0, "records are copied in 16-byte pieces");
-    static_assert(kStride % 2 == 1, "frame rows must start in different banks");
-    // Per-frame masks (mode kRaw): a byte per slot, frame rows an odd number
-    // of words apart (32 lanes reading one slot of their frames hit 32 banks).
-    static constexpr int kMStride = 4 * (((DCAP + 4) / 4) | 1);
-    // Entry pairs: A, then B (spread, masks), then C (spread).
-    template <int MODE>
-    static constexpr size_t pair_bytes() {
-        return MODE == kSpread ? 40 : MODE == kRaw ? 32 : 16;
-    }
-    template <int MODE>
-    static constexpr size_t buf_bytes() {
-        return size_t(kFrames) * kStride * 4 + size_t(PCAP) * pair_bytes<MODE>() +
-               (MODE == kRaw ? size_t(kFrames) * kMStride : 0);
-    }
-    // Buffers, records, then the mbarriers: full[BUFS], empty[BUFS], record[kMetaBufs].
-    template <int MODE>
-    static constexpr size_t bar_offset() {
-        return size_t(BUFS) * buf_bytes<MODE>() + size_t(kMetaBufs) * kMetaWords * 4;
-    }
-    template <int MODE>
-    static constexpr size_t smem_bytes() {
-        return bar_offset<MODE>() + size_t(2 * BUFS + kMetaBufs) * 8;
-    }
-};
-// Mapping 8's layout can be changed at build time for measurements
-// (-DDG_BT8_ROWS=24, -DDG_BT8_DCAP=128 -DDG_BT8_PCAP=200 -DDG_BT8_BUFS=4 -DDG_BT8_AHEAD=2).
-#ifndef DG_BT8_ROWS
-#define DG_BT8_ROWS 16
-#endif
-#ifndef DG_BT8_DCAP
-#define DG_BT8_DCAP 160
-#endif
-#ifndef DG_BT8_PCAP
-#define DG_BT8_PCAP 256
-#endif
-#ifndef DG_BT8_BUFS
-#define DG_BT8_BUFS 3
-#endif
-#ifndef DG_BT8_AHEAD
-#define DG_BT8_AHEAD 1
-#endif
-// 2-byte pixels of the bin tiles loaded with a chunk's copies and stored
-// after the chunk before it is summed (1), or stored as they arrive (0).
-#ifndef DG_BT_DEFER_PX
-#define DG_BT_DEFER_PX 1
-#endif
-// With two frames per lane, the lane's two frames stored side by side in
-// shared memory (1: one 8-byte load per slot) or in separate frame rows (0).
-#ifndef DG_BT_PAIRED
-#define DG_BT_PAIRED 0
-#endif
-// Shared-memory addresses of the bin tiles' pixel copies and pixel loads
-// kept as 32-bit integers (1) or left to the compiler (0).
-#ifndef DG_BT_SADDR
-#define DG_BT_SADDR 1
-#endif
-// Bin-tile sums per (row, frame): packed FP32 partials folded into an FP64
-// sum (1) or into double-word FP32 sums (0).
-#ifndef DG_BT_ACC64
-#define DG_BT_ACC64 1
-#endif
-using BtAcc = std::conditional<DG_BT_ACC64 != 0, AccP64, Acc2>::type;
-// Mapping 8's neighbouring tiles launched as 2-CTA clusters (1) or one CTA
-// per tile (0).
-#ifndef DG_BT_CLUSTER_PAIRS
-#define DG_BT_CLUSTER_PAIRS 0
-#endif
-// Bin tiles run largest first (1) or in bin order (0).
-#ifndef DG_BT_LARGEST_FIRST
-#define DG_BT_LARGEST_FIRST 1
-#endif
-// Pairs of a row summed in plain FP32 (each half of a packed accumulator
-// takes one entry per pair) before they are folded into the double-word sums.
-#ifndef DG_BT_FOLD_PAIRS
-#define DG_BT_FOLD_PAIRS 32
-#endif
-constexpr int kBtFoldPairs = DG_BT_FOLD_PAIRS;
-constexpr bool kBtClusterPairs = DG_BT_CLUSTER_PAIRS != 0;
-using Bt7 = BtCfg<24, 384, 640, 1, 4>;  // mapping 7
-using Bt8 = BtCfg<DG_BT8_ROWS, DG_BT8_DCAP, DG_BT8_PCAP, 2, (DG_BT8_ROWS > 16 ? 2 : 4),
-                  DG_BT8_BUFS, DG_BT8_AHEAD>;  // mapping 8
-static_assert(Bt7::smem_bytes<kSpread>() <= 227 * 1024, "mapping 7 fits shared memory");
-static_assert(Bt8::smem_bytes<kSpread>() <= 227 * 1024, "mapping 8 fits shared memory");
-// Per-frame masks on mapping 8's tiles (same rows and chunks, so the same
-// records): one frame per lane leaves registers for the four sums.
-// Two frames per lane for 4-byte pixels (the FP64 folds leave the registers
-// for four sums of two frames: 76 k against 72 k frames/s on the Eiger-4M
-// batch); 2-byte pixels, whose mask and pixel loads are deferred in
-// registers, keep one.
-template <typename P>
-using BtR = BtCfg<DG_BT8_ROWS, DG_BT8_DCAP, DG_BT8_PCAP, sizeof(P) == 2 ? 1 : 2, 4, DG_BT8_BUFS,
-                  DG_BT8_AHEAD>;
-static_assert(BtR<float>::kMetaWords == Bt8::kMetaWords &&
-                  BtR<uint16_t>::kMetaWords == Bt8::kMetaWords &&
-                  BtR<float>::kMetaHead == Bt8::kMetaHead,
-              "masked tiles read mapping 8's chunk records");
-static_assert(BtR<float>::smem_bytes<kRaw>() <= 227 * 1024 &&
-                  BtR<uint16_t>::smem_bytes<kRaw>() <= 227 * 1024,
-              "masked tiles fit shared memory");
-
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-    const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-
-// Shared-memory mbarriers of the bin-tile chunk pipeline.
-__device__ __forceinline__ unsigned smem_addr(const void *p) {
-    return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t *b, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(b)), "r"(count)
-                 : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *b) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_addr(b)) : "memory");
-}
-// Arrives (without raising the expected count) once all of this thread's
-// earlier cp.async copies have landed.
-__device__ __forceinline__ void mbar_arrive_copies(uint64_t *b) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_addr(b))
-                 : "memory");
-}
-// Waits for the phase of the given parity to complete; gives up (false)
-// after kBtWaitNs of global time, so a lost arrival cannot hang the GPU.
-// (A suspend-time hint on the try, 1 ms, measured 2% slower on mapping 8.)
-constexpr uint64_t kBtWaitNs = 1000000000ull;
-// Tries between two reads of the global timer, and the pause (ns) after a
-// failed try (0: none), of a waiting warp.
-#ifndef DG_BT_WAIT_TRIES
-#define DG_BT_WAIT_TRIES 1
-#endif
-#ifndef DG_BT_WAIT_SLEEP
-#define DG_BT_WAIT_SLEEP 0
-#endif
-__device__ __forceinline__ bool mbar_try(unsigned a, unsigned parity) {
-    unsigned done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    return done != 0;
-}
-__device__ __forceinline__ uint64_t global_ns() {
-    uint64_t now;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-    return now;
-}
-__device__ __forceinline__ bool mbar_wait(uint64_t *b, unsigned parity) {
-    const unsigned a = smem_addr(b);
-    if (mbar_try(a, parity)) return true;
-    const uint64_t t0 = global_ns();
-    for (;;) {
-#pragma unroll 1
-        for (int n = 0; n < DG_BT_WAIT_TRIES; ++n) {
-            if (DG_BT_WAIT_SLEEP > 0) __nanosleep(DG_BT_WAIT_SLEEP);
-            if (mbar_try(a, parity)) return true;
-        }
-        if (global_ns() - t0 > kBtWaitNs) return false;
-    }
-}
-
-template <int MODE, typename P, class CFG>
-__global__ void __launch_bounds__(CFG::kThreads, 1)
-    k_gather_bins(const int4 *__restrict__ items, const int32_t *__restrict__ meta,
-                  const float4 *__restrict__ pair_a, const float4 *__restrict__ pair_b,
-                  const float2 *__restrict__ pair_c,
-                  const int4 *__restrict__ org, const float4 *__restrict__ entry_std,
-                  const double *__restrict__ den, const double *__restrict__ den_std,
-                  const int32_t *__restrict__ valid_std,
-                  const P *__restrict__ frames, int64_t n_pixels, int n_frames, int n_rows,
-                  double *__restrict__ out_i, double *__restrict__ out_s,
-                  double *__restrict__ out_d, int *__restrict__ wait_err, int withhold,
-                  const double *__restrict__ raw_cnt, double *__restrict__ out_c, int raw,
-                  const uint8_t *__restrict__ masks, int64_t mask_stride, int paired) {
-    using S = StagedPx<P>;
-    constexpr int NA = NAcc<MODE, P>::value;
-    constexpr bool SPREAD = MODE == kSpread;
-    constexpr int F2 = CFG::kF2, STRIDE = CFG::kStride, DCAP = CFG::kDCap, PCAP = CFG::kPCap;
-    // Float pixels with the spread keep five sums per frame (the excluded
-    // non-finite weights): half the unroll keeps them in registers.
-#ifndef DG_BT_FLOAT_SPREAD_U2
-#define DG_BT_FLOAT_SPREAD_U2 2
-#endif
-    constexpr int U2 = (SPREAD && is_float_px<P>() && CFG::kU2 > DG_BT_FLOAT_SPREAD_U2)
-                           ? DG_BT_FLOAT_SPREAD_U2
-                           : CFG::kU2;
-    constexpr int NT = CFG::kThreads, NW = CFG::kRows;
-    constexpr int NB = CFG::kBufs, NM = CFG::kMetaBufs, AH = CFG::kAhead, MA = CFG::kMetaAhead;
-    constexpr int MH = CFG::kMetaHead, MW = CFG::kMetaWords;
-    constexpr size_t BUF = CFG::template buf_bytes<MODE>();
-    constexpr bool WIDE = SPREAD || MODE == kRaw;  // 32-byte entry pairs
-    constexpr int MS = CFG::kMStride;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int groups = (n_frames + CFG::kFrames - 1) / CFG::kFrames;
-    // Paired tiles: the two CTAs of a cluster take neighbouring tiles 2m and
-    // 2m + 1 for the same frames.
-    int item_idx, group;
-    if (paired) {
-        const int per = 2 * groups, m = int(blockIdx.x) / per, rm = int(blockIdx.x) % per;
-        item_idx = 2 * m + (rm & 1);
-        group = rm >> 1;
-    } else {
-        item_idx = int(blockIdx.x) / groups;
-        group = int(blockIdx.x) % groups;
-    }
-    const int4 it = items[item_idx];
-    const int f0 = group * CFG::kFrames;
-    const int nv = min(CFG::kFrames, n_frames - f0);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int row0 = it.x, nrows = it.y, ch0 = it.z, nch = it.w;
-    // Failure-detection check (dg_plan_test_wait_timeout): warp 0 of the first
-    // CTA never reports a chunk summed, so the waits for its buffers run out.
-    const bool signal = !(withhold && blockIdx.x == 0 && warp == 0);
-
-    auto pxbuf = [&](int b) { return reinterpret_cast<S *>(smem + size_t(b) * BUF); };
-    // Staged pixel of (local frame f, slot k). With two frames per lane the
-    // lane's frames l and l + 32 can sit side by side (PAIRED: one 8-byte
-    // shared load reads a slot for both; rows of 2 * STRIDE words, STRIDE odd,
-    // so the 16 lanes of a half-warp hit 16 distinct bank pairs).
-    constexpr bool PAIRED = DG_BT_PAIRED && F2 == 2 && MODE != kRaw;
-    auto pxi = [&](int f, int k) {
-        return PAIRED ? (f & 31) * 2 * STRIDE + 2 * k + (f >> 5) : f * STRIDE + k;
-    };
-    auto pabuf = [&](int b) {
-        return reinterpret_cast<float4 *>(smem + size_t(b) * BUF +
-                                          size_t(CFG::kFrames) * STRIDE * 4);
-    };
-    auto mbuf = [&](int c) {
-        return reinterpret_cast<int32_t *>(smem + size_t(NB) * BUF) + (c % NM) * MW;
-    };
-    auto mkbuf = [&](int b) {  // mask rows (mode kRaw)
-        return smem + size_t(b) * BUF + size_t(CFG::kFrames) * STRIDE * 4 + size_t(PCAP) * 32;
-    };
-    auto pcbuf = [&](int b) {  // pairs C (spread)
-        return reinterpret_cast<f2 *>(smem + size_t(b) * BUF + size_t(CFG::kFrames) * STRIDE * 4 +
-                                      size_t(PCAP) * 32);
-    };
-    // full[b]: chunk in buffer b landed (every thread's copies and stores);
-    // empty[b]: every warp has summed the chunk in buffer b; rec[m]: the
-    // record in slot m landed.
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + CFG::template bar_offset<MODE>());
-    uint64_t *empty = full + NB, *rec = full + 2 * NB;
-    if (tid == 0) {
-        for (int b = 0; b < NB; ++b) {
-            mbar_init(full + b, NT);
-            mbar_init(empty + b, NW);
-        }
-        for (int m = 0; m < NM; ++m) mbar_init(rec + m, NT);
-    }
-    // Column DCAP of every frame row is read by padding pairs and holds 0.
-    for (int j = tid; j < NB * CFG::kFrames; j += NT) {
-        pxbuf(j / CFG::kFrames)[pxi(j % CFG::kFrames, DCAP)] = S(0);
-        if constexpr (MODE == kRaw) mkbuf(j / CFG::kFrames)[(j % CFG::kFrames) * MS + DCAP] = 0;
-    }
-    __syncthreads();
-
-    // Copy chunk c's record into its slot; every thread arrives on the
-    // slot's barrier once its copies have landed (all threads arriving, not
-    // only the copying ones, measured faster: 2.03 against 2.67 ms).
-    auto stage_meta = [&](int c) {
-        const int4 *src = reinterpret_cast<const int4 *>(meta + int64_t(ch0 + c) * MW);
-        int4 *dst = reinterpret_cast<int4 *>(mbuf(c));
-        for (int j = tid; j < MW / 4; j += NT) cp_async16(dst + j, src + j);
-        mbar_arrive_copies(rec + c % NM);
-    };
-    // Stage chunk c into buffer c % NB (its record is in shared memory); every
-    // thread arrives on the buffer's full barrier, counted once its copies
-    // have landed and ordering its plain stores (2-byte pixels) before it.
-    // Mode kRaw: a chunk's mask bytes, loaded with its copies and stored into
-    // shared memory only after the warp has summed the chunk before it, so
-    // the loads' latency hides behind that work.
-    constexpr int KS = CFG::kSlices, FS = CFG::kStageFrames, FSTEP = CFG::kRows / KS;
-    constexpr int KSTEP = ((DCAP + KS - 1) / KS + 31) / 32;
-    unsigned mv[MODE == kRaw ? KSTEP : 1][FS];
-    // 2-byte pixels are loaded, not copied: their loads are deferred the same
-    // way where the registers allow it (512 threads, no spread).
-    constexpr bool DEFER_PX = DG_BT_DEFER_PX && sizeof(P) != 4 && MODE != kSpread && NT <= 512;
-    constexpr bool DEFER = MODE == kRaw || DEFER_PX;
-    S pv[DEFER_PX ? KSTEP : 1][FS];
-    // The first of two halves of staging chunk c: mask loads and copies.
-    // The frames this warp stages (4-byte pixels), found once per tile.
-    const P *stage_frame[FS];
-    const uint64_t l2pol = bt_l2_policy();
-#pragma unroll
-    for (int j = 0; j < FS; ++j)
-        stage_frame[j] = frames + int64_t(f0 + min(warp / KS + j * FSTEP, max(nv - 1, 0))) * n_pixels;
-    auto stage_issue = [&](int c, int b) {  // b = c % NB
-        const int32_t *mb = mbuf(c);
-        const int4 ch = make_int4(0, mb[0], mb[2], mb[1]);  // {-, pixels, first pair, pairs}
-        const int per = (ch.y + KS - 1) / KS, s0 = (warp % KS) * per;
-        const int k1 = min(ch.y, s0 + per), fw = warp / KS;
-        S *dst = pxbuf(b);
-        const P *base = frames + int64_t(f0 + fw) * n_pixels;
-        if constexpr (MODE == kRaw) {
-#pragma unroll
-            for (int i = 0; i < KSTEP; ++i) {
-                const int k = s0 + lane + 32 * i;
-#pragma unroll
-                for (int j = 0; j < FS; ++j) {
-                    const int f = fw + j * FSTEP;
-                    mv[i][j] = k < k1 && f < nv
-                                   ? unsigned(__ldg(masks + int64_t(f0 + f) * mask_stride + mb[MH + k]))
-                                   : 0u;
-                }
-            }
-        }
-        if constexpr (DEFER_PX) {
-#pragma unroll
-            for (int i = 0; i < KSTEP; ++i) {
-                const int k = s0 + lane + 32 * i;
-#pragma unroll
-                for (int j = 0; j < FS; ++j)
-                    pv[i][j] = k < k1 && fw + j * FSTEP < nv
-                                   ? load_px<P>(base + mb[MH + k] + int64_t(j * FSTEP) * n_pixels, 0u)
-                                   : S(0);
-            }
-        } else if constexpr (sizeof(P) == 4) {
-            // This lane's slots s0 + lane + 32 i and their pixel indices, read
-            // once; then frame by frame, one address add and one copy per
-            // (slot, frame).
-            uint32_t boff[KSTEP];  // byte offsets of the slots' pixels in a frame
-            bool kin[KSTEP];
-#pragma unroll
-            for (int i = 0; i < KSTEP; ++i) {
-                const int k = s0 + lane + 32 * i;
-                kin[i] = k < k1;
-                boff[i] = kin[i] ? uint32_t(mb[MH + k]) * uint32_t(sizeof(P)) : 0u;
-            }
-#pragma unroll
-            for (int j = 0; j < FS; ++j) {
-                const int f = fw + j * FSTEP;
-                if (f >= nv) break;
-#if DG_BT_SADDR
-                const char *fsrc = reinterpret_cast<const char *>(stage_frame[j]);
-                const unsigned drow = smem_addr(dst + pxi(f, s0 + lane));
-                constexpr unsigned kStep = 4u * (PAIRED ? 64u : 32u);  // 32 slots on
-#pragma unroll
-                for (int i = 0; i < KSTEP; ++i)
-                    if (kin[i]) cp_async4_sp(drow + kStep * unsigned(i), fsrc + boff[i], l2pol);
-#else
-                const P *fsrc = base + int64_t(j * FSTEP) * n_pixels;
-                int idx[KSTEP];
-#pragma unroll
-                for (int i = 0; i < KSTEP; ++i) idx[i] = int(boff[i] / uint32_t(sizeof(P)));
-#pragma unroll
-                for (int i = 0; i < KSTEP; ++i)
-                    if (kin[i]) cp_async4(dst + pxi(f, s0 + lane + 32 * i), fsrc + idx[i]);
-#endif
-            }
-        } else {
-            for (int k = s0 + lane; k < k1; k += 32) {
-                const P *src = base + mb[MH + k];
-#pragma unroll
-                for (int j = 0; j < FS; ++j) {
-                    if (fw + j * FSTEP >= nv) break;
-                    dst[pxi(fw + j * FSTEP, k)] = load_px<P>(src + int64_t(j * FSTEP) * n_pixels, 0u);
-                }
-            }
-        }
-        float4 *pa = pabuf(b);
-        f2 *pc = pcbuf(b);
-        for (int j = tid; j < ch.w; j += NT) {
-            cp_async16(pa + j, pair_a + ch.z + j);
-            if (WIDE) cp_async16(pa + PCAP + j, pair_b + ch.z + j);
-            if (SPREAD) cp_async8(pc + j, pair_c + ch.z + j);
-        }
-    };
-    // The second half: mask stores, then this thread's arrival on the
-    // buffer's full barrier.
-    auto stage_finish = [&](int c, int b) {
-        if constexpr (DEFER_PX) {
-            const int dn = mbuf(c)[0];
-            const int per = (dn + KS - 1) / KS, s0 = (warp % KS) * per;
-            const int k1 = min(dn, s0 + per), fw = warp / KS;
-            S *dst = pxbuf(b);
-#pragma unroll
-            for (int i = 0; i < KSTEP; ++i) {
-                const int k = s0 + lane + 32 * i;
-#pragma unroll
-                for (int j = 0; j < FS; ++j)
-                    if (k < k1 && fw + j * FSTEP < nv) dst[pxi(fw + j * FSTEP, k)] = pv[i][j];
-            }
-        }
-        if constexpr (MODE == kRaw) {
-            const int32_t *mb = mbuf(c);
-            const int dn = mb[0];
-            const int per = (dn + KS - 1) / KS, s0 = (warp % KS) * per;
-            const int k1 = min(dn, s0 + per), fw = warp / KS;
-            unsigned char *md = mkbuf(b);
-#pragma unroll
-            for (int i = 0; i < KSTEP; ++i) {
-                const int k = s0 + lane + 32 * i;
-#pragma unroll
-                for (int j = 0; j < FS; ++j) {
-                    const int f = fw + j * FSTEP;
-                    if (k < k1 && f < nv) md[f * MS + k] = static_cast<unsigned char>(mv[i][j]);
-                }
-            }
-        }
-        asm volatile("cp.async.mbarrier.arrive.shared::cta.b64 [%0];\n" ::"r"(smem_addr(full + b))
-                     : "memory");
-        mbar_arrive(full + b);
-    };
-    auto stage = [&](int c, int b) {
-        stage_issue(c, b);
-        stage_finish(c, b);
-    };
-
-    // This warp's row: accumulators, fold counter and origin of each of the
-    // lane's frames.
-    BtAcc acc[F2][NA];
-#pragma unroll
-    for (int h = 0; h < F2; ++h)
-#pragma unroll
-        for (int a = 0; a < NA; ++a) acc[h][a].zero();
-    int since = 0;
-    const int r = warp;  // row of the tile
-    // Origin of the spread's shift, per frame of the lane: the row's origin
-    // entry {origin, first valid, row end} read from the frames before the
-    // first chunk (row_origin).
-    float orgv[F2];
-#pragma unroll
-    for (int h = 0; h < F2; ++h) orgv[h] = 0.f;
-    if constexpr (SPREAD) {
-        if (r < nrows) {
-            const int4 o = org[row0 + r];
-#pragma unroll
-            for (int h = 0; h < F2; ++h) {
-                const int fi = min(f0 + lane + 32 * h, n_frames - 1);
-                orgv[h] = row_origin<P>(entry_std, o.x, o.y, o.z, frames + int64_t(fi) * n_pixels);
-            }
-        }
-    }
-    f2 norg[F2];
-#pragma unroll
-    for (int h = 0; h < F2; ++h) norg[h] = pk(-orgv[h], -orgv[h]);
-
-    // Pipeline without a CTA-wide barrier: in step c a warp stages its share
-    // of chunk c + AH (once every warp has summed the chunk that buffer held)
-    // and of record c + AH + MA, then sums chunk c once all its shares have
-    // landed. A warp may fall kLag chunks behind the fastest, so rows whose
-    // entries are unevenly spread over the chunks even out over the tile.
-    bool ok = true;
-    for (int j = 0; j < AH + MA && j < nch; ++j) stage_meta(j);
-    static_assert(AH < NB, "the first chunks go to buffers 0..AH-1");
-    for (int j = 0; j < AH && j < nch; ++j) {
-        if (ok) ok = mbar_wait(rec + j % NM, unsigned(j / NM) & 1u);
-        if (ok) stage(j, j);
-    }
-    // Buffers and phases of chunks c and j = c + AH, kept as counters (c % NB
-    // and c / NB without a division per chunk).
-    int cb = 0, cq = 0, jb = AH, jq = 0;
-    for (int c = 0; c < nch; ++c) {
-        const int j = c + AH;
-        bool pending = false;  // chunk j's second staging half, after chunk c
-        if (j < nch) {
-            if (ok && j >= NB) ok = mbar_wait(empty + jb, unsigned(jq - 1) & 1u);
-            if (ok && j + MA < nch) stage_meta(j + MA);
-            if (ok) ok = mbar_wait(rec + j % NM, unsigned(j / NM) & 1u);
-            if (ok) {
-                if constexpr (DEFER) {
-                    stage_issue(j, jb);
-                    pending = true;
-                } else {
-                    stage(j, jb);
-                }
-            }
-        }
-        if (ok) ok = mbar_wait(full + cb, unsigned(cq) & 1u);
-        if (!__all_sync(0xffffffffu, ok)) {
-            ok = false;
-            break;
-        }
-        const int b = cb, pb = jb;  // pb: chunk j's buffer, for its second half
-        if (++cb == NB) {
-            cb = 0;
-            ++cq;
-        }
-        if (++jb == NB) {
-            jb = 0;
-            ++jq;
-        }
-        if (r >= nrows) {
-            if (pending) stage_finish(j, pb);
-            if (lane == 0 && signal) mbar_arrive(empty + b);
-            continue;
-        }
-        const S *px[F2];
-        unsigned pxa[F2];  // the same as 32-bit shared-memory addresses
-#pragma unroll
-        for (int h = 0; h < F2; ++h) {
-            px[h] = pxbuf(b) + pxi(lane + 32 * h, 0);
-            pxa[h] = smem_addr(px[h]);
-        }
-        const float4 *s_pa = pabuf(b);
-        const float4 *s_pb = s_pa + PCAP;
-        const f2 *s_pc = pcbuf(b);
-        const unsigned char *mk[F2];  // this lane's mask rows (mode kRaw)
-#pragma unroll
-        for (int h = 0; h < F2; ++h) mk[h] = mkbuf(b) + (lane + 32 * h) * MS;
-        const int32_t *cp = mbuf(c) + 4;
-        const int p0 = cp[r], p1 = cp[r + 1];
-        auto body = [&](int p, auto unroll) {
-            constexpr int UU = decltype(unroll)::value;
-            float4 ea[UU], eb[UU];
-            f2 ec[UU];
-#pragma unroll
-            for (int u = 0; u < UU; ++u) {
-                ea[u] = s_pa[p + u];
-                if constexpr (WIDE) eb[u] = s_pb[p + u];
-                if constexpr (SPREAD) ec[u] = s_pc[p + u];
-            }
-            // the pair's pixels for this lane's frames
-            float vv0[F2][UU], vv1[F2][UU];
-            if constexpr (PAIRED) {
-#pragma unroll
-                for (int u = 0; u < UU; ++u) {
-                    using S2 = typename std::conditional<std::is_same<S, float>::value, float2,
-                               typename std::conditional<std::is_same<S, int32_t>::value, int2,
-                                                         uint2>::type>::type;
-                    const S2 a = *reinterpret_cast<const S2 *>(px[0] + 2 * __float_as_int(ea[u].x));
-                    const S2 b2 = *reinterpret_cast<const S2 *>(px[0] + 2 * __float_as_int(ea[u].y));
-                    vv0[0][u] = float(a.x);
-                    vv0[F2 - 1][u] = float(a.y);
-                    vv1[0][u] = float(b2.x);
-                    vv1[F2 - 1][u] = float(b2.y);
-                }
-            } else if constexpr (DG_BT_SADDR && MODE != kRaw) {
-#pragma unroll
-                for (int h = 0; h < F2; ++h)
-#pragma unroll
-                    for (int u = 0; u < UU; ++u) {
-                        vv0[h][u] = staged_value<S>(
-                            lds32(pxa[h] + 4u * unsigned(__float_as_int(ea[u].x))));
-                        vv1[h][u] = staged_value<S>(
-                            lds32(pxa[h] + 4u * unsigned(__float_as_int(ea[u].y))));
-                    }
-            } else {
-#pragma unroll
-                for (int h = 0; h < F2; ++h)
-#pragma unroll
-                    for (int u = 0; u < UU; ++u) {
-                        vv0[h][u] = float(px[h][__float_as_int(ea[u].x)]);
-                        vv1[h][u] = float(px[h][__float_as_int(ea[u].y)]);
-                    }
-            }
-#pragma unroll
-            for (int h = 0; h < F2; ++h) {
-                float(&v0)[UU] = vv0[h];
-                float(&v1)[UU] = vv1[h];
-                if constexpr (MODE == kRaw) {
-                    // Per-frame masks: {slot, slot, w, w}, {w*norm, w*norm, 0, 0};
-                    // a masked entry adds nothing to S, V, N or C, whatever its
-                    // pixel holds.
-#pragma unroll
-                    for (int u = 0; u < UU; ++u) {
-                        const bool l0 = mk[h][__float_as_int(ea[u].x)] == 0;
-                        const bool l1 = mk[h][__float_as_int(ea[u].y)] == 0;
-                        const f2 cc = pk(l0 ? ea[u].z : 0.f, l1 ? ea[u].w : 0.f);
-                        const float x0 = l0 ? v0[u] : 0.f, x1 = l1 ? v1[u] : 0.f;
-                        const f2 x = pk(x0, x1);
-                        acc[h][0].p = fma2(cc, x, acc[h][0].p);
-                        const f2 xp = is_unsigned_px<P>() ? x : pk(fmaxf(x0, 0.f), fmaxf(x1, 0.f));
-                        acc[h][1].p = fma2(mul2(cc, cc), xp, acc[h][1].p);
-                        acc[h][2].p = add2(acc[h][2].p, pk(l0 ? eb[u].x : 0.f, l1 ? eb[u].y : 0.f));
-                        acc[h][3].p = add2(acc[h][3].p, cc);
-                    }
-                    continue;
-                }
-#pragma unroll
-                for (int u = 0; u < UU; ++u) {
-                    const f2 cc = pk(ea[u].z, ea[u].w);
-                    if constexpr (SPREAD && is_float_px<P>()) {
-                        if (!(isfinite(v0[u]) && isfinite(v1[u]))) {
-                            const bool ok0 = isfinite(v0[u]), ok1 = isfinite(v1[u]);
-                            const float x0 = ok0 ? v0[u] : 0.f, x1 = ok1 ? v1[u] : 0.f;
-                            const f2 ce = pk(ok0 ? ea[u].z : 0.f, ok1 ? ea[u].w : 0.f);
-                            const f2 x = pk(x0, x1), n = pk(eb[u].x, eb[u].y);
-                            const f2 cre = pk(ok0 ? eb[u].z : 0.f, ok1 ? eb[u].w : 0.f);
-                            acc[h][0].p = fma2(ce, x, acc[h][0].p);
-                            acc[h][1].p = fma2(mul2(ce, ce), pk(fmaxf(x0, 0.f), fmaxf(x1, 0.f)),
-                                               acc[h][1].p);
-                            const f2 t = fma2(norg[h], ec[u], fma2(norg[h], n, x));
-                            acc[h][2].p = fma2(mul2(cre, t), t, acc[h][2].p);
-                            acc[h][kSpreadA].p = fma2(ce, t, acc[h][kSpreadA].p);
-                            acc[h][NA - 2].p = add2(acc[h][NA - 2].p,
-                                                    pk(ok0 ? 0.f : __fmul_rn(ea[u].z, eb[u].x),
-                                                       ok1 ? 0.f : __fmul_rn(ea[u].w, eb[u].y)));
-                            acc[h][NA - 1].p = add2(acc[h][NA - 1].p,
-                                                    pk(!ok0 && ea[u].z > 0.f ? 1.f : 0.f,
-                                                       !ok1 && ea[u].w > 0.f ? 1.f : 0.f));
-                            continue;
-                        }
-                    }
-                    const f2 x = pk(v0[u], v1[u]);
-                    acc[h][0].p = fma2(cc, x, acc[h][0].p);
-                    if constexpr (MODE != kIntensity) {
-                        const f2 xp = is_unsigned_px<P>()
-                                          ? x
-                                          : pk(fmaxf(v0[u], 0.f), fmaxf(v1[u], 0.f));
-                        acc[h][1].p = fma2(mul2(cc, cc), xp, acc[h][1].p);
-                    }
-                    if constexpr (SPREAD) {
-                        const f2 n = pk(eb[u].x, eb[u].y), cr = pk(eb[u].z, eb[u].w);
-                        const f2 t = fma2(norg[h], ec[u], fma2(norg[h], n, x));
-                        acc[h][2].p = fma2(mul2(cr, t), t, acc[h][2].p);
-                        acc[h][kSpreadA].p = fma2(cc, t, acc[h][kSpreadA].p);
-                    }
-                }
-            }
-        };
-        auto fold = [&]() {
-#pragma unroll
-            for (int h = 0; h < F2; ++h)
-#pragma unroll
-                for (int a = 0; a < NA; ++a) acc[h][a].flush();
-        };
-        int p = p0;
-        for (; p + U2 <= p1; p += U2) {
-            body(p, std::integral_constant<int, U2>{});
-            since += U2;
-            if (since >= kBtFoldPairs) {
-                since = 0;
-                fold();
-            }
-        }
-        for (; p < p1; ++p) {
-            body(p, std::integral_constant<int, 1>{});
-            if (++since >= kBtFoldPairs) {
-                since = 0;
-                fold();
-            }
-        }
-        if (pending) stage_finish(j, pb);
-        __syncwarp();
-        if (lane == 0 && signal) mbar_arrive(empty + b);
-    }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    if (!ok) {
-        // A wait gave up: this tile's sums are incomplete. The host finds the
-        // flag (mapped host memory) and reports the call as failed.
-        if (lane == 0) {
-            *reinterpret_cast<volatile int *>(wait_err) = 1;
-            __threadfence_system();
-        }
-        return;
-    }
-    if (r >= nrows) return;
-
-    // Normalise (normalize_bin, prepared.rs:985-996; the spread's closing
-    // formulas, azimuthal.rs:96-104), as k_finalize does from partial sums.
-#pragma unroll
-    for (int h = 0; h < F2; ++h) {
-        const int fl = lane + 32 * h;
-        if (fl >= nv) continue;
-        const int row = row0 + r;
-        double v[NA];
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-            acc[h][a].flush();
-            v[a] = acc[h][a].value();
-        }
-        const int64_t oo = int64_t(f0 + fl) * n_rows + row;
-        if constexpr (MODE == kRaw) {
-            // Sums of this frame's mask: raw (integrate1d_raw*) or normalised
-            // by the frame's own N (normalize_bin), as k_finalize_raw and
-            // k_finalize<kRaw> do from partial sums.
-            if (raw) {
-                out_i[oo] = v[0];
-                out_d[oo] = v[2];
-                if (out_s) out_s[oo] = v[1];
-                out_c[oo] = v[3];
-            } else {
-                const double n = v[2];
-                out_i[oo] = n == 0.0 ? 0.0 : v[0] / n;
-                if (out_s) {
-                    const double q = n == 0.0 ? 0.0 : v[1] / (n * n);
-                    out_s[oo] = sqrt(q > 0.0 ? q : 0.0);
-                }
-            }
-            continue;
-        }
-        if (raw) {
-            // Raw sums (integrate1d_raw*, integrate.rs:682-797): signal and
-            // variance sums of the frame, the row's strict norm and weight sums.
-            out_i[oo] = v[0];
-            if (NA > 1 && out_s) out_s[oo] = v[NA > 1 ? 1 : 0];
-            out_d[oo] = den[row];
-            out_c[oo] = raw_cnt[row];
-            continue;
-        }
-        if constexpr (!SPREAD) {
-            const double n = den[row];
-            out_i[oo] = n == 0.0 ? 0.0 : v[0] / n;
-            if (MODE == kErrors) {
-                const double q = n == 0.0 ? 0.0 : v[1] / (n * n);
-                out_s[oo] = sqrt(q > 0.0 ? q : 0.0);
-            }
-        } else {
-            int valid = valid_std[row];
-            double sw = den_std[row];
-            if (NA == 6) {
-                valid -= int(v[NA - 1] + 0.5);
-                sw -= v[NA - 2];
-            }
-            if (valid <= 0 || !(sw > 0.0)) {
-                out_i[oo] = 0.0;
-                if (out_s) out_s[oo] = 0.0;
-                out_d[oo] = __longlong_as_double(0x7ff8000000000000ll);
-                continue;
-            }
-            const double a1 = v[kSpreadA];
-            out_i[oo] = v[0] / sw;
-            if (out_s) out_s[oo] = sqrt(v[1] > 0.0 ? v[1] : 0.0) / sw;
-            const double mean = a1 / sw;
-            const double m2 = v[2] - mean * a1;
-            const double q = m2 / sw;
-            // one valid contribution: its deviation from itself is exactly 0
-            out_d[oo] = valid == 1 ? 0.0 : sqrt(q > 0.0 ? q : 0.0);
-        }
-    }
-}
-
-// Bin-tile entry pairs from the plan-time layout: per pair {slot 0, slot 1,
-// entry 0, entry 1} (entry -1: padding, slot = the zero column) to A {slot 0, slot 1,
-// c0, c1} with the table's FP32 weights, AS the same with the spread's
-// weights, B {n0, n1, c0/n0, c1/n1}.
-__global__ void k_bt_fill(const int4 *__restrict__ desc, int64_t n_pairs,
-                          const int2 *__restrict__ entry, const float4 *__restrict__ entry_std,
-                          const float *__restrict__ entry_nlo, float4 *__restrict__ pair_a,
-                          float4 *__restrict__ pair_as, float4 *__restrict__ pair_b,
-                          float2 *__restrict__ pair_c) {
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n_pairs;
-         i += int64_t(gridDim.x) * blockDim.x) {
-        const int4 d = desc[i];
-        float c[2] = {0.f, 0.f}, cs[2] = {0.f, 0.f}, n[2] = {1.f, 1.f}, cr[2] = {0.f, 0.f},
-              nlo[2] = {0.f, 0.f};
-        const int k[2] = {d.z, d.w};
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (k[h] < 0) continue;
-            c[h] = __int_as_float(entry[k[h]].y);
-            const float4 es = entry_std[k[h]];
-            cs[h] = es.y;
-            n[h] = es.z;
-            cr[h] = es.w;
-            nlo[h] = entry_nlo[k[h]];
-        }
-        pair_a[i] = make_float4(__int_as_float(d.x), __int_as_float(d.y), c[0], c[1]);
-        pair_as[i] = make_float4(__int_as_float(d.x), __int_as_float(d.y), cs[0], cs[1]);
-        pair_b[i] = make_float4(n[0], n[1], cr[0], cr[1]);
-        pair_c[i] = make_float2(nlo[0], nlo[1]);
-    }
-}
-
-// Pairs of the per-frame-mask bin tiles from the same layout: A {slot 0,
-// slot 1, w0, w1} and B {w0*norm, w1*norm, 0, 0} with the raw entries'
-// FP32 weights (k_pack_raw); padding entries are zero.
-__global__ void k_bt_fill_raw(const int4 *__restrict__ desc, int64_t n_pairs,
-                              const float4 *__restrict__ entry_raw, float4 *__restrict__ pair_a,
-                              float4 *__restrict__ pair_b) {
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n_pairs;
-         i += int64_t(gridDim.x) * blockDim.x) {
-        const int4 d = desc[i];
-        float w[2] = {0.f, 0.f}, wn[2] = {0.f, 0.f};
-        const int k[2] = {d.z, d.w};
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (k[h] < 0) continue;
-            const float4 e = entry_raw[k[h]];
-            w[h] = e.y;
-            wn[h] = e.z;
-        }
-        pair_a[i] = make_float4(__int_as_float(d.x), __int_as_float(d.y), w[0], w[1]);
-        pair_b[i] = make_float4(wn[0], wn[1], 0.f, 0.f);
-    }
-}
-
 // One thread per (frame, row): fold the row's segment partials in strip
 // order in FP64 and normalise (normalize_bin, prepared.rs:985-996; the
 // spread's closing formulas, azimuthal.rs:96-104).
@@ -2563,51 +1538,23 @@ void launch_fl(const GatherTable &t, const P *fp, int64_t n_pixels, int nf, doub
 
 // Launches lane-mapping variant `variant` of the gather (kVariantCount) with
 // its partial sums in `partial`.
-template <int MODE, typename P, class CFG>
-void launch_bins(const GatherTable &t, const BinTiles &bt, const P *fp, int64_t n_pixels, int nf,
-                 double *oi, double *os, double *od, cudaStream_t s, double *oc = nullptr,
-                 int raw = 0, const uint8_t *masks = nullptr, int64_t mask_stride = 0) {
-    constexpr size_t smem = CFG::template smem_bytes<MODE>();
-    auto kern = k_gather_bins<MODE, P, CFG>;
-    DG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    const int groups = (nf + CFG::kFrames - 1) / CFG::kFrames;
-    const int64_t grid = int64_t(bt.n_items) * groups;
-    if (grid > INT32_MAX) fail(DG_UNSUPPORTED, "too many bin tiles for one launch");
-    check_bin_tile_waits(t);
-    const float4 *pa = MODE == kSpread ? bt.pair_as.ptr : MODE == kRaw ? bt.pair_ra.ptr : bt.pair_a.ptr;
-    const float4 *pb = MODE == kRaw ? bt.pair_rb.ptr : bt.pair_b.ptr;
-    const int paired = bt.paired ? 1 : 0;
-    if (!paired) {
-        kern<<<unsigned(grid), CFG::kThreads, smem, s>>>(
-            bt.item.ptr, bt.meta.ptr, pa, pb, bt.pair_c.ptr, bt.org.ptr, t.entry_std.ptr,
-            t.den.ptr, t.den_std.ptr, t.valid_std.ptr, fp, n_pixels, nf, t.n_rows, oi, os, od,
-            bt.wait_err.dev, t.withhold_test, t.cnt.ptr, oc, raw, masks, mask_stride, paired);
-        return;
-    }
-    // one 2-CTA cluster per (tile pair, frame group): both CTAs on one GPC
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(unsigned(grid), 1, 1);
-    lc.blockDim = dim3(CFG::kThreads, 1, 1);
-    lc.dynamicSmemBytes = smem;
-    lc.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
-    DG_CUDA(cudaLaunchKernelEx(&lc, kern, static_cast<const int4 *>(bt.item.ptr),
-                               static_cast<const int32_t *>(bt.meta.ptr), pa, pb,
-                               static_cast<const float2 *>(bt.pair_c.ptr),
-                               static_cast<const int4 *>(bt.org.ptr),
-                               static_cast<const float4 *>(t.entry_std.ptr),
-                               static_cast<const double *>(t.den.ptr),
-                               static_cast<const double *>(t.den_std.ptr),
-                               static_cast<const int32_t *>(t.valid_std.ptr), fp, n_pixels, nf,
-                               int(t.n_rows), oi, os, od, bt.wait_err.dev, t.withhold_test,
-                               static_cast<const double *>(t.cnt.ptr), oc, raw, masks,
-                               mask_stride, paired));
+template <int MODE, typename P>
+void launch_finalize(const GatherTable &t, const double *partial, int nf, double *oi, double *os,
+                     double *od, cudaStream_t s) {
+    const dim3 grid(unsigned((t.n_rows + kFinRows - 1) / kFinRows), unsigned((nf + 31) / 32));
+    k_finalize<MODE, P><<<grid, 32 * kFinRows, 0, s>>>(partial, t.row_seg.ptr, t.seg_ids.ptr,
+                                                        t.den.ptr, t.den_std.ptr, t.valid_std.ptr,
+                                                        t.n_rows, nf, oi, os, od);
+    DG_CUDA(cudaGetLastError());
+}
+
+template <typename P>
+constexpr int dtype_code() {
+    return std::is_same<P, uint16_t>::value   ? DG_U16
+           : std::is_same<P, uint32_t>::value ? DG_U32
+           : std::is_same<P, int32_t>::value  ? DG_I32
+           : std::is_same<P, float>::value    ? DG_F32
+                                              : DG_F64;
 }
 
 // Row warps (mapping 10): F frames per pass over a row's entries, one CTA
@@ -2631,7 +1578,7 @@ void launch_rows(const GatherTable &t, const P *fp, int64_t n_pixels, int nf, do
 // partial sums for k_finalize. Those mappings need the outputs; callers without
 // them (raw sums) get the frame-lane or an entry-lane mapping instead.
 template <int MODE, typename P>
-bool launch_gather(const GatherTable &t, int variant, const P *fp, int64_t n_pixels, int nf,
+bool launch_gather(GatherTable &t, int variant, const P *fp, int64_t n_pixels, int nf,
                    double *partial, cudaStream_t s, const uint8_t *masks = nullptr,
                    int64_t mask_stride = 0, double *oi = nullptr, double *os = nullptr,
                    double *od = nullptr) {
@@ -2646,11 +1593,18 @@ bool launch_gather(const GatherTable &t, int variant, const P *fp, int64_t n_pix
             variant = 2;
         }
         if (variant == 7 || variant == 8) {
-            const BinTiles &bt = t.bt[variant - 7];
-            if (oi && bt.n_items > 0) {
-                if (variant == 7) launch_bins<MODE, P, Bt7>(t, bt, fp, n_pixels, nf, oi, os, od, s);
-                else launch_bins<MODE, P, Bt8>(t, bt, fp, n_pixels, nf, oi, os, od, s);
-                DG_CUDA(cudaGetLastError());
+            if (oi && t.bt[variant - 7].n_items > 0) {
+                BinCall c{};
+                c.frames = fp;
+                c.dtype = dtype_code<P>();
+                c.mode = MODE;
+                c.n_pixels = n_pixels;
+                c.n_frames = nf;
+                c.out_i = oi;
+                c.out_s = os;
+                c.out_d = od;
+                c.partial = partial;
+                launch_bin_tiles(t, variant, c, s);
                 return true;
             }
             variant = t.fl_n_units > 0 ? 5 : 2;
@@ -2681,7 +1635,7 @@ bool launch_gather(const GatherTable &t, int variant, const P *fp, int64_t n_pix
 }
 
 template <typename P>
-bool launch_typed(const GatherTable &t, int variant, const void *frames, int64_t n_pixels,
+bool launch_typed(GatherTable &t, int variant, const void *frames, int64_t n_pixels,
                   int n_frames, int mode, double *partial, double *oi, double *os, double *od,
                   cudaStream_t s) {
     const P *fp = static_cast<const P *>(frames);
@@ -2695,16 +1649,6 @@ bool launch_typed(const GatherTable &t, int variant, const void *frames, int64_t
                                         0, oi, os, od);
 }
 
-template <int MODE, typename P>
-void launch_finalize(const GatherTable &t, const double *partial, int nf, double *oi, double *os,
-                     double *od, cudaStream_t s) {
-    const dim3 grid(unsigned((t.n_rows + kFinRows - 1) / kFinRows), unsigned((nf + 31) / 32));
-    k_finalize<MODE, P><<<grid, 32 * kFinRows, 0, s>>>(partial, t.row_seg.ptr, t.seg_ids.ptr,
-                                                        t.den.ptr, t.den_std.ptr, t.valid_std.ptr,
-                                                        t.n_rows, nf, oi, os, od);
-    DG_CUDA(cudaGetLastError());
-}
-
 template <typename P>
 void finalize_typed(const GatherTable &t, int mode, const double *partial, int nf, double *oi,
                     double *os, double *od, cudaStream_t s) {
@@ -2714,6 +1658,13 @@ void finalize_typed(const GatherTable &t, int mode, const double *partial, int n
 }
 
 }  // namespace
+
+int sm_count() {
+    int dev = 0, sms = 0;
+    DG_CUDA(cudaGetDevice(&dev));
+    DG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    return std::max(1, sms);
+}
 
 int gather_launches_per_call() { return 2; }
 
@@ -2845,308 +1796,6 @@ void build_fl_units(GatherTable &out, const DeviceCsr &table, const std::vector<
     DG_CUDA(cudaStreamSynchronize(s));
     out.fl_pair_as = own_spread ? out.fl_pair_s.ptr : out.fl_pair_a.ptr;
     out.fl_n_units = int32_t(fl.size());
-}
-
-// Bin tiles (k_gather_bins) at plan time, on the host: for every run of
-// CFG::kRows rows, the rows' entries merged in pixel order and cut into chunks of
-// at most kBtDCap distinct pixels and kBtPCap pairs (a new pixel that would
-// exceed either opens the next chunk, so a chunk is a pixel-index interval
-// and each row's entries in it are a contiguous run of its CSR row). Tiles
-// are ordered largest first. Each row keeps {origin entry, first valid entry,
-// row end} for the spread's origin (row_origin), read before the first chunk.
-template <class CFG>
-void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cudaStream_t s) {
-    constexpr int kBtDCap = CFG::kDCap, kBtPCap = CFG::kPCap, kBtRows = CFG::kRows;
-    constexpr int kBtMetaHead = CFG::kMetaHead, kBtMetaWords = CFG::kMetaWords;
-    const int64_t nb = table.n_rows;
-    out.n_items = 0;
-    if (nb == 0 || table.nnz == 0) return;
-    out.wait_err.alloc();
-    std::vector<int64_t> rp(static_cast<size_t>(nb) + 1);
-    DG_CUDA(cudaMemcpyAsync(rp.data(), table.row_ptr.ptr, rp.size() * 8, cudaMemcpyDeviceToHost, s));
-    std::vector<int32_t> col(static_cast<size_t>(table.nnz)), fv(static_cast<size_t>(nb)),
-        oe(static_cast<size_t>(nb));
-    DG_CUDA(cudaMemcpyAsync(col.data(), table.col.ptr, col.size() * 4, cudaMemcpyDeviceToHost, s));
-    DG_CUDA(cudaMemcpyAsync(fv.data(), gt.first_valid.ptr, fv.size() * 4, cudaMemcpyDeviceToHost, s));
-    DG_CUDA(cudaMemcpyAsync(oe.data(), gt.origin.ptr, oe.size() * 4, cudaMemcpyDeviceToHost, s));
-    DG_CUDA(cudaStreamSynchronize(s));
-    const int64_t n_items = (nb + kBtRows - 1) / kBtRows;
-    struct Tile {
-        std::vector<int4> chunks;      // {px offset, D, pair offset, pairs} (tile-relative)
-        std::vector<int32_t> cpair;    // per chunk kBtRows + 1
-        std::vector<int32_t> px;
-        std::vector<int4> pairs;       // {slot0, slot1, entry0, entry1}
-        int64_t entries = 0;
-    };
-    std::vector<Tile> tiles(static_cast<size_t>(n_items));
-    auto build = [&](int64_t ti) {
-        Tile &T = tiles[size_t(ti)];
-        const int64_t r0 = ti * kBtRows, r1 = std::min<int64_t>(nb, r0 + kBtRows);
-        const int nr = int(r1 - r0);
-        // Entries merged in pixel order, rows ascending within a pixel: keys
-        // pixel << 32 | row << 27 | position in row; each row is sorted
-        // already, so four rounds of pairwise merges order the tile.
-        const int64_t n_e = rp[size_t(r1)] - rp[size_t(r0)];
-        std::vector<uint64_t> ka(static_cast<size_t>(n_e)), kb(static_cast<size_t>(n_e));
-        std::vector<int64_t> bounds(static_cast<size_t>(kBtRows) + 1, 0);
-        for (int j = 0; j < nr; ++j) {
-            const int64_t b = rp[size_t(r0 + j)], e = rp[size_t(r0 + j) + 1];
-            if (e - b >= (int64_t(1) << 27)) fail(DG_UNSUPPORTED, "a bin too large for bin tiles");
-            uint64_t *o = ka.data() + (b - rp[size_t(r0)]);
-            for (int64_t k = b; k < e; ++k)
-                o[k - b] = (uint64_t(uint32_t(col[size_t(k)])) << 32) | (uint64_t(j) << 27) |
-                           uint64_t(k - b);
-            bounds[size_t(j) + 1] = e - rp[size_t(r0)];
-        }
-        for (int j = nr; j < kBtRows; ++j) bounds[size_t(j) + 1] = n_e;
-        for (int width = 1; width < kBtRows; width *= 2) {
-            for (int j = 0; j < kBtRows; j += 2 * width) {
-                const int64_t a0 = bounds[size_t(j)], a1 = bounds[size_t(std::min(j + width, kBtRows))],
-                              a2 = bounds[size_t(std::min(j + 2 * width, kBtRows))];
-                std::merge(ka.begin() + a0, ka.begin() + a1, ka.begin() + a1, ka.begin() + a2,
-                           kb.begin() + a0);
-            }
-            ka.swap(kb);
-        }
-        struct Ent {
-            int32_t px, row, k;
-        };
-        std::vector<Ent> m(static_cast<size_t>(n_e));
-        for (int64_t i = 0; i < n_e; ++i) {
-            const uint64_t key = ka[size_t(i)];
-            const int j = int((key >> 27) & 31u);
-            m[size_t(i)] = {int32_t(key >> 32), j, int32_t(rp[size_t(r0 + j)] + int64_t(key & ((1u << 27) - 1)))};
-        }
-        T.entries = n_e;
-        T.pairs.reserve(size_t(n_e / 2 + 64));
-        T.px.reserve(size_t(n_e / 2 + 64));
-        std::vector<std::vector<std::pair<int32_t, int32_t>>> run(static_cast<size_t>(nr));  // (slot, entry)
-        std::vector<int32_t> chunk_px;
-        auto close = [&]() {
-            if (chunk_px.empty()) return;
-            int4 ch = make_int4(int(T.px.size()), int(chunk_px.size()), int(T.pairs.size()), 0);
-            T.px.insert(T.px.end(), chunk_px.begin(), chunk_px.end());
-            int po = 0;
-            for (int j = 0; j < kBtRows; ++j) {
-                T.cpair.push_back(po);
-                if (j >= nr) continue;
-                const auto &rv = run[size_t(j)];
-                for (size_t e = 0; e < rv.size(); e += 2) {
-                    const bool two = e + 1 < rv.size();
-                    T.pairs.push_back(make_int4(rv[e].first, two ? rv[e + 1].first : kBtDCap,
-                                                rv[e].second, two ? rv[e + 1].second : -1));
-                    ++po;
-                }
-            }
-            T.cpair.push_back(po);
-            ch.w = po;
-            T.chunks.push_back(ch);
-            chunk_px.clear();
-            for (auto &rv : run) rv.clear();
-        };
-        int pairs = 0;
-        for (size_t i = 0; i < m.size();) {
-            size_t e = i;
-            while (e < m.size() && m[e].px == m[i].px) ++e;
-            // pairs after adding this pixel's entries
-            int add = 0;
-            for (size_t q = i; q < e; ++q) add += (run[size_t(m[q].row)].size() % 2 == 0) ? 1 : 0;
-            if (!chunk_px.empty() &&
-                (int(chunk_px.size()) + 1 > kBtDCap || pairs + add > kBtPCap)) {
-                close();
-                pairs = 0;
-                add = int(e - i);
-            }
-            const int slot = int(chunk_px.size());
-            chunk_px.push_back(m[i].px);
-            for (size_t q = i; q < e; ++q) run[size_t(m[q].row)].push_back({slot, m[q].k});
-            pairs += add;
-            i = e;
-        }
-        close();
-    };
-    const int nt = int(std::min<int64_t>(
-        n_items, std::max(1u, std::min(16u, std::thread::hardware_concurrency()))));
-    auto parallel = [&](auto &&fn, int64_t count) {
-        std::vector<std::thread> pool;
-        std::atomic<int64_t> next{0};
-        for (int t = 0; t < nt; ++t)
-            pool.emplace_back([&]() {
-                for (int64_t i; (i = next.fetch_add(1)) < count;) fn(i);
-            });
-        for (auto &th : pool) th.join();
-    };
-    parallel(build, n_items);
-    // Tile order, then flatten.
-    std::vector<int64_t> order(static_cast<size_t>(n_items));
-    for (int64_t i = 0; i < n_items; ++i) order[size_t(i)] = i;
-#if DG_BT_LARGEST_FIRST
-    std::stable_sort(order.begin(), order.end(), [&](int64_t a, int64_t b) {
-        return tiles[size_t(a)].entries > tiles[size_t(b)].entries;
-    });
-#endif
-    // Mapping 8: neighbouring tiles 2m, 2m + 1 side by side (pairs largest
-    // first), launched as 2-CTA clusters so both run on one GPC and read the
-    // pixel runs they share through the same L2; -1 marks the empty partner
-    // of an odd last tile.
-    out.paired = false;
-    if (kBtClusterPairs && std::is_same<CFG, Bt8>::value && n_items > 1) {
-        const int64_t np = (n_items + 1) / 2;
-        std::vector<int64_t> pairs_order(static_cast<size_t>(np));
-        auto pair_size = [&](int64_t m) {
-            int64_t e = tiles[size_t(2 * m)].entries;
-            if (2 * m + 1 < n_items) e = std::max<int64_t>(e, tiles[size_t(2 * m + 1)].entries);
-            return e;
-        };
-        for (int64_t m = 0; m < np; ++m) pairs_order[size_t(m)] = m;
-        std::stable_sort(pairs_order.begin(), pairs_order.end(),
-                         [&](int64_t a, int64_t b) { return pair_size(a) > pair_size(b); });
-        order.clear();
-        for (int64_t m : pairs_order) {
-            order.push_back(2 * m);
-            order.push_back(2 * m + 1 < n_items ? 2 * m + 1 : -1);
-        }
-        out.paired = true;
-    }
-    const int64_t n_slots = int64_t(order.size());
-    // Output offsets of every tile, then the tiles copied in parallel.
-    std::vector<int64_t> o_ch(size_t(n_slots) + 1, 0), o_px(size_t(n_slots) + 1, 0),
-        o_pr(size_t(n_slots) + 1, 0);
-    const Tile empty_tile;
-    auto tile_at = [&](int64_t i) -> const Tile & {
-        return order[size_t(i)] < 0 ? empty_tile : tiles[size_t(order[size_t(i)])];
-    };
-    for (int64_t i = 0; i < n_slots; ++i) {
-        const Tile &T = tile_at(i);
-        o_ch[size_t(i) + 1] = o_ch[size_t(i)] + int64_t(T.chunks.size());
-        o_px[size_t(i) + 1] = o_px[size_t(i)] + int64_t(T.px.size());
-        o_pr[size_t(i) + 1] = o_pr[size_t(i)] + int64_t(T.pairs.size());
-    }
-    if (o_pr[size_t(n_slots)] > INT32_MAX || o_px[size_t(n_slots)] > INT32_MAX)
-        fail(DG_UNSUPPORTED, "table too large for bin tiles");
-    // default-initialised (not zeroed): every element is written below
-    const size_t n_chunks = size_t(o_ch[size_t(n_slots)]), n_pairs = size_t(o_pr[size_t(n_slots)]);
-    std::vector<int4> items(static_cast<size_t>(n_slots)), org(static_cast<size_t>(nb));
-    // per row {origin entry, first valid entry, row end, 0} (row_origin)
-    for (int64_t r = 0; r < nb; ++r)
-        org[size_t(r)] = make_int4(oe[size_t(r)], fv[size_t(r)], int(rp[size_t(r) + 1]), 0);
-    std::unique_ptr<int32_t[]> meta(new int32_t[std::max<size_t>(n_chunks * kBtMetaWords, 1)]);
-    std::unique_ptr<int4[]> pairs(new int4[std::max<size_t>(n_pairs, 1)]);
-    auto flatten = [&](int64_t i) {
-        const int64_t ti = order[size_t(i)];
-        if (ti < 0) {  // the empty partner: no rows, no chunks
-            items[size_t(i)] = make_int4(0, 0, int(o_ch[size_t(i)]), 0);
-            return;
-        }
-        Tile &T = tiles[size_t(ti)];
-        const int64_t c0 = o_ch[size_t(i)], pr0 = o_pr[size_t(i)];
-        for (size_t c = 0; c < T.chunks.size(); ++c) {
-            const int4 ch = T.chunks[c];
-            int32_t *rec = meta.get() + (size_t(c0) + c) * kBtMetaWords;
-            rec[0] = ch.y;
-            rec[1] = ch.w;
-            rec[2] = int32_t(ch.z + pr0);
-            rec[3] = 0;
-            for (int j = 0; j < kBtMetaHead - 4; ++j)
-                rec[4 + j] = j <= kBtRows ? T.cpair[c * (kBtRows + 1) + size_t(j)] : 0;
-            std::copy(T.px.begin() + ch.x, T.px.begin() + ch.x + ch.y, rec + kBtMetaHead);
-            std::fill(rec + kBtMetaHead + ch.y, rec + kBtMetaWords, 0);
-        }
-        std::copy(T.pairs.begin(), T.pairs.end(), pairs.get() + pr0);
-        const int64_t r0 = ti * kBtRows;
-        const int nr = int(std::min<int64_t>(nb, r0 + kBtRows) - r0);
-        items[size_t(i)] = make_int4(int(r0), nr, int(c0), int(T.chunks.size()));
-        T = Tile();
-    };
-    parallel(flatten, n_slots);
-    out.n_items = int32_t(items.size());
-    out.item.alloc(items.size());
-    out.meta.alloc(std::max<size_t>(n_chunks * kBtMetaWords, 1));
-    out.org.alloc(org.size());
-    out.pair_a.alloc(std::max<size_t>(n_pairs, 1));
-    out.pair_as.alloc(std::max<size_t>(n_pairs, 1));
-    out.pair_b.alloc(std::max<size_t>(n_pairs, 1));
-    out.pair_c.alloc(std::max<size_t>(n_pairs, 1));
-    DeviceArray<int4> &desc = out.desc;  // kept for the per-frame-mask pairs
-    desc.alloc(std::max<size_t>(n_pairs, 1));
-    out.pair_ra.release();
-    out.pair_rb.release();
-    out.raw_built = false;
-    DG_CUDA(cudaMemcpyAsync(out.item.ptr, items.data(), items.size() * sizeof(int4),
-                            cudaMemcpyHostToDevice, s));
-    if (n_chunks)
-        DG_CUDA(cudaMemcpyAsync(out.meta.ptr, meta.get(), n_chunks * kBtMetaWords * 4,
-                                cudaMemcpyHostToDevice, s));
-    DG_CUDA(cudaMemcpyAsync(out.org.ptr, org.data(), org.size() * sizeof(int4),
-                            cudaMemcpyHostToDevice, s));
-    if (n_pairs) {
-        DG_CUDA(cudaMemcpyAsync(desc.ptr, pairs.get(), n_pairs * sizeof(int4),
-                                cudaMemcpyHostToDevice, s));
-        k_bt_fill<<<148 * 8, 256, 0, s>>>(desc.ptr, int64_t(n_pairs), gt.entry.ptr,
-                                         gt.entry_std.ptr, gt.entry_nlo.ptr, out.pair_a.ptr,
-                                         out.pair_as.ptr, out.pair_b.ptr, out.pair_c.ptr);
-        DG_CUDA(cudaGetLastError());
-    }
-    DG_CUDA(cudaStreamSynchronize(s));
-    // Only mapping 8's tiles carry per-frame masks (BtR); the others drop the
-    // descriptor once their pairs are filled.
-    if (!std::is_same<CFG, Bt8>::value) desc.release();
-}
-
-namespace {
-__global__ void k_flip_meta(int32_t *__restrict__ meta, int64_t n_rec, int words, int head,
-                            int rows, int cols);
-}  // namespace
-
-bool bin_tile_wait_failed(const GatherTable &t) {
-    bool failed = false;
-    for (const BinTiles &bt : t.bt)
-        if (bt.wait_err.host && *static_cast<volatile int *>(bt.wait_err.host)) {
-            *bt.wait_err.host = 0;
-            failed = true;
-        }
-    return failed;
-}
-
-void check_bin_tile_waits(const GatherTable &t) {
-    if (bin_tile_wait_failed(t))
-        fail(DG_TIMEOUT, "bin-tile gather: a chunk-pipeline wait gave up after 1 s; the "
-                          "results of a launch on this plan since the last check are invalid");
-}
-
-void ensure_bin_tiles(GatherTable &t, const DeviceCsr &table, int variant, cudaStream_t s) {
-    if (variant != 7 && variant != 8) return;
-    BinTiles &bt = t.bt[variant - 7];
-    if (bt.built) return;
-    AllocScope alloc(s);  // s is synchronised before this returns
-    int words = 0, head = 0;
-    if (variant == 7) {
-        build_bin_tiles<Bt7>(t, bt, table, s);
-        words = Bt7::kMetaWords;
-        head = Bt7::kMetaHead;
-    } else {
-        build_bin_tiles<Bt8>(t, bt, table, s);
-        words = Bt8::kMetaWords;
-        head = Bt8::kMetaHead;
-    }
-    if (t.flip_rows && bt.n_items > 0) {
-        k_flip_meta<<<148 * 4, 256, 0, s>>>(bt.meta.ptr, int64_t(bt.meta.count) / words, words,
-                                            head, t.flip_rows, t.flip_cols);
-        DG_CUDA(cudaGetLastError());
-        DG_CUDA(cudaStreamSynchronize(s));
-    }
-    bt.built = true;
-}
-
-bool gather_variant_needs_tiles(int variant) { return variant == 7 || variant == 8; }
-
-bool bin_tiles_fill_gpu(const GatherTable &t, int variant, int64_t n_frames) {
-    if (!gather_variant_needs_tiles(variant)) return false;
-    const int64_t rows = variant == 7 ? Bt7::kRows : Bt8::kRows;
-    const int64_t per = variant == 7 ? Bt7::kFrames : Bt8::kFrames;
-    const int64_t nf = std::min<int64_t>(n_frames, 256);
-    const int64_t ctas = (int64_t(t.n_rows) + rows - 1) / rows * ((nf + per - 1) / per);
-    return 2 * nf >= per && ctas >= 2 * 148;
 }
 
 void make_gather_table(const DeviceCsr &table, const double *d_norm, int32_t dim1, int32_t dim2,
@@ -3312,13 +1961,24 @@ bool gather_writes_results(const GatherTable &t) {
     return (t.variant == 7 || t.variant == 8) && t.bt[t.variant - 7].n_items > 0;
 }
 
+int64_t partial_rows(const GatherTable &t) {
+    if (t.n_units == 0) return 0;
+    if (gather_writes_results(t)) return t.variant == 10 ? 0 : bin_tile_partials(t, t.variant);
+    return std::max<int64_t>(1, t.n_segments);
+}
+
 void reserve_partials(GatherTable &t, int64_t n_frames, uint32_t flags, int dtype,
                       bool any_mapping) {
-    if ((!any_mapping && gather_writes_results(t)) || n_frames <= 0) return;
+    if (n_frames <= 0) return;
     const int mode = (flags & DG_AZIMUTHAL_STD) ? kSpread : (flags & DG_ERRORS) ? kErrors
                                                                                 : kIntensity;
-    const int64_t need = std::max<int64_t>(1, t.n_segments) *
-                         n_accumulators(mode, dtype == DG_F32 || dtype == DG_F64) *
+    int64_t rows = partial_rows(t);
+    if (any_mapping) {
+        rows = std::max<int64_t>(1, t.n_segments);
+        for (int v : {7, 8})
+            if (t.bt[v - 7].n_items > 0) rows = std::max(rows, bin_tile_partials(t, v));
+    }
+    const int64_t need = rows * n_accumulators(mode, dtype == DG_F32 || dtype == DG_F64) *
                          std::min<int64_t>(256, (n_frames + 31) / 32 * 32);
     if (t.partial.count < size_t(need)) t.partial.alloc(size_t(need));
 }
@@ -3442,10 +2102,7 @@ void run_gather(GatherTable &t, const void *d_frames, int dtype, int64_t n_pixel
     double *partial = nullptr;
     if (scratch) {
         const bool fpx = dtype == DG_F32 || dtype == DG_F64;
-        const int64_t per_frame =
-            gather_writes_results(t) || t.n_units == 0
-                ? 0
-                : std::max<int64_t>(1, t.n_segments) * n_accumulators(mode, fpx);
+        const int64_t per_frame = partial_rows(t) * n_accumulators(mode, fpx);
         if (per_frame > 0) chunk = std::min<int64_t>(chunk, int64_t(scratch_doubles) / per_frame);
         if (chunk < 1)
             fail(DG_UNSUPPORTED, "this plan needs " + std::to_string(per_frame * 8) +
@@ -3454,11 +2111,16 @@ void run_gather(GatherTable &t, const void *d_frames, int dtype, int64_t n_pixel
         partial = scratch;
     } else {
         // [segment][accumulator][frame] for the largest launch of this call,
-        // frames rounded up to 32 so that growing batches reallocate rarely
-        reserve_partials(t, std::min<int64_t>(chunk, n_frames), flags, dtype, true);
-        t.scratch.wait(s);
+        // frames rounded up to 32 so that growing batches reallocate rarely;
+        // mappings without partial sums do not allocate them
+        if (partial_rows(t) > 0)
+            reserve_partials(t, std::min<int64_t>(chunk, n_frames), flags, dtype);
         partial = t.partial.ptr;
     }
+    // The plan's partial sums and the bin tiles' item counter are shared by its
+    // calls; row warps share nothing.
+    const bool shared = gather_variant_needs_tiles(t.variant) || (!scratch && partial_rows(t) > 0);
+    if (shared) t.scratch.wait(s);
     const size_t esize = dtype == DG_U16 ? 2 : dtype == DG_F64 ? 8 : 4;
     for (int64_t f0 = 0; f0 < n_frames; f0 += chunk) {
         const int nf = int(std::min<int64_t>(chunk, n_frames - f0));
@@ -3501,7 +2163,7 @@ void run_gather(GatherTable &t, const void *d_frames, int dtype, int64_t n_pixel
             }
         }
     }
-    if (!scratch) t.scratch.mark(s);
+    if (shared) t.scratch.mark(s);
 }
 
 namespace {
@@ -3517,12 +2179,6 @@ __global__ void k_flip_px_norm(float2 *__restrict__ a, int rows, int cols) {
         a[i] = a[j];
         a[j] = t;
     }
-}
-
-// Row flip of a pixel index for frames stored bottom row first.
-__device__ __forceinline__ int32_t flip_px(int32_t j, int rows, int cols) {
-    const int32_t r = j / cols, c = j - r * cols;
-    return (rows - 1 - r) * cols + c;
 }
 
 // InputOrder::FlipVertical: every pixel index the gathers load through,
@@ -3541,17 +2197,6 @@ __global__ void k_flip_rows(int2 *__restrict__ entry, float4 *__restrict__ entry
             const int32_t v = px[i - nnz];
             if (v >= 0 && v < npix) px[i - nnz] = flip_px(v, rows, cols);
         }
-    }
-}
-
-// The same for the pixel indices of bin-tile chunk records (D of them each).
-__global__ void k_flip_meta(int32_t *__restrict__ meta, int64_t n_rec, int words, int head,
-                            int rows, int cols) {
-    for (int64_t r = blockIdx.x; r < n_rec; r += gridDim.x) {
-        int32_t *rec = meta + r * words;
-        const int d = rec[0];
-        for (int k = threadIdx.x; k < d; k += blockDim.x)
-            rec[head + k] = flip_px(rec[head + k], rows, cols);
     }
 }
 
@@ -3596,35 +2241,26 @@ bool launch_raw(GatherTable &t, const void *frames, int64_t n_pixels, int nf, in
                 const uint8_t *masks, int64_t mask_stride, cudaStream_t s, bool raw, double *o0,
                 double *o1, double *o2, double *o3) {
     const P *fp = static_cast<const P *>(frames);
-    // Per-frame masks on a mapping-8 plan: the masked tiles write the raw
-    // sums (S, N, V, C in o0..o3) or the normalised results (o0, o1).
-    if (mode == kRaw && t.variant == 8 && t.bt[1].n_items > 0 && t.entry_raw.ptr) {
-        BinTiles &bt = t.bt[1];
-        if (!bt.raw_built) {
-            bt.pair_ra.alloc(bt.desc.count);
-            bt.pair_rb.alloc(bt.desc.count);
-            k_bt_fill_raw<<<148 * 8, 256, 0, s>>>(bt.desc.ptr, int64_t(bt.desc.count),
-                                                 t.entry_raw.ptr, bt.pair_ra.ptr, bt.pair_rb.ptr);
-            DG_CUDA(cudaGetLastError());
-            bt.raw_built = true;
-        }
-        if (raw) launch_bins<kRaw, P, BtR<P>>(t, bt, fp, n_pixels, nf, o0, o2, o1, s, o3, 1, masks, mask_stride);
-        else launch_bins<kRaw, P, BtR<P>>(t, bt, fp, n_pixels, nf, o0, o1, nullptr, s, nullptr, 0, masks, mask_stride);
-        DG_CUDA(cudaGetLastError());
-        return true;
-    }
-    // Raw sums over the plan mask on a bin-tile plan: the tiles write them.
-    if (raw && mode != kRaw && gather_variant_needs_tiles(t.variant) &&
+    // Per-frame masks on a mapping-8 plan (raw sums S, N, V, C in o0..o3, or the
+    // normalised results in o0, o1), and raw sums over the plan mask on a
+    // bin-tile plan: the tiles take them.
+    if ((mode == kRaw ? t.variant == 8 && t.entry_raw.ptr : raw && gather_variant_needs_tiles(t.variant)) &&
         t.bt[t.variant - 7].n_items > 0) {
-        const BinTiles &bt = t.bt[t.variant - 7];
-        if (mode == kErrors) {
-            if (t.variant == 7) launch_bins<kErrors, P, Bt7>(t, bt, fp, n_pixels, nf, o0, o2, o1, s, o3, 1);
-            else launch_bins<kErrors, P, Bt8>(t, bt, fp, n_pixels, nf, o0, o2, o1, s, o3, 1);
-        } else {
-            if (t.variant == 7) launch_bins<kIntensity, P, Bt7>(t, bt, fp, n_pixels, nf, o0, nullptr, o1, s, o3, 1);
-            else launch_bins<kIntensity, P, Bt8>(t, bt, fp, n_pixels, nf, o0, nullptr, o1, s, o3, 1);
-        }
-        DG_CUDA(cudaGetLastError());
+        BinCall c{};
+        c.frames = frames;
+        c.dtype = dtype_code<P>();
+        c.mode = mode;
+        c.n_pixels = n_pixels;
+        c.n_frames = nf;
+        c.out_i = o0;
+        c.out_s = raw ? o2 : o1;
+        c.out_d = raw ? o1 : nullptr;
+        c.out_c = raw ? o3 : nullptr;
+        c.raw = raw ? 1 : 0;
+        c.masks = masks;
+        c.mask_stride = mask_stride;
+        c.partial = t.partial.ptr;
+        launch_bin_tiles(t, t.variant, c, s);
         return true;
     }
     if (mode == kRaw)
@@ -3647,8 +2283,10 @@ void run_gather_raw(GatherTable &t, const void *d_frames, int dtype, int64_t n_p
     const bool errors = (flags & DG_ERRORS) != 0;
     const int mode = d_masks ? kRaw : errors ? kErrors : kIntensity;
     const int64_t chunk = 256;
-    const int64_t need = std::max<int64_t>(1, t.n_segments) *
-                         n_accumulators(mode, dtype == DG_F32 || dtype == DG_F64) *
+    int64_t rows = std::max<int64_t>(1, t.n_segments);
+    for (int v : {7, 8})
+        if (t.bt[v - 7].n_items > 0) rows = std::max(rows, bin_tile_partials(t, v));
+    const int64_t need = rows * n_accumulators(mode, dtype == DG_F32 || dtype == DG_F64) *
                          std::min<int64_t>(chunk, (n_frames + 31) / 32 * 32);
     if (t.partial.count < size_t(need)) t.partial.alloc(size_t(need));
     t.scratch.wait(s);

@@ -246,15 +246,21 @@ struct EventPool {
     }
 };
 
-// One bin-tile layout (dg_gather.cu): runs of rows whose entries are cut
+// One bin-tile layout (dg_bins.cu): runs of rows whose entries are cut
 // into pixel-interval chunks, built on first use.
 struct BinTiles {
     bool built = false;
     int32_t n_items = 0;
     DeviceArray<int4> item;        // {first row, rows, first chunk, chunks}, largest first
-    // Items 2m and 2m + 1 are neighbouring tiles launched as one 2-CTA
-    // cluster per frame group (an odd count ends with an empty item).
-    bool paired = false;
+    // Large tiles cut into pieces (items): per item and row the {chunk, pair}
+    // it starts and ends at, for both fold cadences, and every row's partial
+    // sums (item * rows + row of the tile) in order.
+    bool split = false;
+    DeviceArray<int32_t> counter;  // a launch's next claim and finished CTAs
+    DeviceArray<int4> span[2];
+    DeviceArray<int32_t> row_part, part_ids;
+    DeviceArray<int32_t> tile_done;     // pieces done per (tile, frame group) of a launch
+    mutable bool unfinished = false;    // a launch gave up: counters to reset
     DeviceArray<int32_t> meta;     // per chunk: {pixels, pairs, first pair}, row offsets, pixels
     DeviceArray<int4> org;         // per row {origin entry, first valid entry, row end, 0}
     DeviceArray<float4> pair_a, pair_as, pair_b;
@@ -267,7 +273,8 @@ struct BinTiles {
     // Set by k_gather_bins when a wait of its chunk pipeline gave up.
     PinnedFlag wait_err;
     int64_t bytes() const {
-        return int64_t(item.bytes() + meta.bytes() + org.bytes() + pair_a.bytes() +
+        return int64_t(span[0].bytes() + span[1].bytes() + row_part.bytes() + part_ids.bytes() + tile_done.bytes() + counter.bytes() +
+                       item.bytes() + meta.bytes() + org.bytes() + pair_a.bytes() +
                        pair_as.bytes() + pair_b.bytes() + pair_c.bytes() + desc.bytes() + pair_ra.bytes() +
                        pair_rb.bytes());
     }
@@ -315,6 +322,7 @@ struct GatherTable {
     // {pixel bits, w, w*norm, 0} per entry and the FP64 weight sum per row.
     DeviceArray<float4> entry_raw;
     DeviceArray<double> cnt;
+    DeviceArray<uint64_t> mask_words;  // scratch: per-frame masks as words (bin tiles)
     // Bin tiles (k_gather_bins), mappings 7 and 8; see dg_gather.cu.
     BinTiles bt[2];
     // Row warps (k_rows), mapping 10: row pointers, rows with more than
@@ -355,9 +363,29 @@ void run_gather(GatherTable &t, const void *d_frames, int dtype, int64_t n_pixel
                 int64_t n_frames, uint32_t flags, int precision, double *d_i, double *d_sigma,
                 double *d_std, cudaStream_t stream, double *scratch = nullptr,
                 size_t scratch_doubles = 0);
-// Whether the plan's gather writes the results itself (bin tiles: no partial
-// sums, no finalize).
+// Whether the plan's gather needs no finalize by the caller (bin tiles, which
+// finalize their own partial sums where they have any, and row warps).
 bool gather_writes_results(const GatherTable &t);
+// Partial sums per frame and accumulator that the plan's mapping leaves.
+int64_t partial_rows(const GatherTable &t);
+// One launch of the bin tiles (dg_bins.cu) on up to 256 frames.
+struct BinCall {
+    const void *frames;
+    int dtype, mode;              // mode: Mode of dg_gather_common.cuh
+    int64_t n_pixels;
+    int n_frames;
+    // I, sigma, std; raw: signal, variance, norm, weight sums
+    double *out_i, *out_s, *out_d, *out_c;
+    int raw;
+    const uint8_t *masks;         // per-frame masks (mapping 8)
+    int64_t mask_stride;
+    double *partial;
+};
+void launch_bin_tiles(GatherTable &t, int variant, const BinCall &c, cudaStream_t s);
+// Partial sums per frame and accumulator of bin tiles 7 or 8 (0: none).
+int64_t bin_tile_partials(const GatherTable &t, int variant);
+// Multiprocessors of the current device.
+int sm_count();
 // Allocates the plan's partial sums for launches of up to n_frames frames of
 // this dtype and these flags, ahead of the first call that needs them (not
 // for a plan whose bin tiles need none, unless `any_mapping`).
