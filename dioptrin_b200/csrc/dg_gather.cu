@@ -418,26 +418,34 @@ __global__ void __launch_bounds__(kThreads)
 // the table over its frames; one frame reads every entry once, so what
 // counts there is keeping enough loads in flight and doing nothing else: no
 // staging, no partial sums, no second launch. A row of at most kRowsLong
-// entries is one warp's (eight rows per CTA), a longer one the whole CTA's
-// (largest first, so the long rows start early). Threads stride the row's
-// entries (coalesced), kRowsU of them in flight each, load the pixels of F
-// frames per entry and sum in FP64; the warp (then the CTA's warps in a fixed
-// order) adds the threads' sums by a fixed butterfly and one thread writes the
-// results (normalize_bin, prepared.rs:985-996; the spread's closing formulas,
-// azimuthal.rs:96-104). The spread is shifted by the row's origin as in the
-// other mappings, in FP64: t = s - o*n with n the entry's FP32 pair.
+// entries is one warp's (eight rows per CTA), one of at most kRowsTiny eight
+// lanes' (32 per CTA), a longer one the whole CTA's, an eighth per warp
+// (largest first, so the long rows start early), or in larger launches one
+// warp's, eighth after eighth (rows_group). Lanes stride the entries
+// (coalesced), kRowsU of them in flight each, load the pixels of F
+// frames per entry and sum in FP64; a fixed butterfly adds the lanes' sums, and
+// the eighths are added in order, so a row's bits do not depend on the launch.
+// One thread writes the results (normalize_bin, prepared.rs:985-996; the spread's
+// closing formulas, azimuthal.rs:96-104). The spread is shifted by the row's
+// origin as in the other mappings, in FP64: t = s - o*n with n the entry's FP32
+// pair.
+//
+// What bounds it: the latency of three dependent loads (row record, entry, pixel;
+// 57 % of an Eiger-4M frame's warp cycles waited on them) with 28 to 64 warps per SM.
+// So the record holds all of a row's plan data (it was an item, a row number and
+// two row pointers, in a chain), and the loads past a row's end are made all the
+// same, of its last entry with weight 0: as predicated loads the compiler finished
+// each before it issued the next. Before and now, us: Eiger-4M with the spread, 1 /
+// 2 / 4 / 64 frames 59.5 / 86.0 / 149.7 / 2148 and 53.0 / 69.6 / 121.6 / 1347; 1
+// frame with errors 34.8 and 30.0; Eiger-4M cake 81.9 and 59.4; Eiger-9M
+// intensities, 1 / 64 frames 36.4 / 745 and 29.8 / 596; Pilatus 1M 14.3 and 12.5.
+// Clusters of eight CTAs that share eight rows' pixels in L1 (57 % hits against
+// 6 %) were no faster for one frame (61.9), nor were loads of the next entries
+// ahead (the registers cost a CTA per SM).
 constexpr int kRowsLong = 512;
 constexpr int kRowsTiny = 64;  // rows of at most this many entries take 8 lanes
-#ifndef DG_ROWS_U
-#define DG_ROWS_U 4
-#endif
-constexpr int kRowsU = DG_ROWS_U;
+constexpr int kRowsU = 4;  // entries in flight per thread
 constexpr int kRowsThreads = 256;
-
-template <typename P>
-__device__ __forceinline__ double load_px_d(const P *__restrict__ f, uint32_t i) {
-    return double(__ldg(f + i));
-}
 
 // Butterfly sum over the 32 lanes: every lane ends with the same value (IEEE
 // addition is commutative, so partners compute the same sums).
@@ -453,196 +461,260 @@ __device__ __forceinline__ double group8_sum_d(double v) {
     return v;
 }
 
-// Shared memory of a row-warp CTA: the warps' sums of a long row.
+// Shared memory of a row-warp CTA: the warps' sums of long rows.
 constexpr int kRowsWarps = kRowsThreads / 32;
 using RowsRed = double[kRowsWarps][4 * kMaxAcc];
 
-// One row-warp item of a plan's batch (q.item[k]); every thread of the CTA
-// calls it. F frames per pass over the entries.
+// Writes one row's results of one frame from its sums v.
+template <int MODE, typename P>
+__device__ __forceinline__ void rows_write(const QueuePlan &qp, int row, int frame, const double *v) {
+    constexpr int NA = NAcc<MODE, P>::value;
+    const int64_t oo = int64_t(frame) * qp.n_rows + row;
+    if constexpr (MODE != kSpread) {
+        const double n = qp.den[row];
+        qp.out_i[oo] = n == 0.0 ? 0.0 : v[0] / n;
+        if (MODE == kErrors) {
+            const double s2 = n == 0.0 ? 0.0 : v[1] / (n * n);
+            qp.out_s[oo] = sqrt(s2 > 0.0 ? s2 : 0.0);
+        }
+    } else {
+        int valid = qp.valid_std[row];
+        double sw = qp.den_std[row];
+        if (NA == 6) {
+            valid -= int(v[NA - 1] + 0.5);
+            sw -= v[NA - 2];
+        }
+        if (valid <= 0 || !(sw > 0.0)) {
+            qp.out_i[oo] = 0.0;
+            if (qp.out_s) qp.out_s[oo] = 0.0;
+            qp.out_d[oo] = __longlong_as_double(0x7ff8000000000000ll);
+            return;
+        }
+        const double a1 = v[kSpreadA];
+        qp.out_i[oo] = v[0] / sw;
+        if (qp.out_s) qp.out_s[oo] = sqrt(v[1] > 0.0 ? v[1] : 0.0) / sw;
+        const double mean = a1 / sw;
+        const double q2 = (v[2] - mean * a1) / sw;
+        // one valid contribution: its deviation from itself is exactly 0
+        qp.out_d[oo] = valid == 1 ? 0.0 : sqrt(q2 > 0.0 ? q2 : 0.0);
+    }
+}
+
+// The row's origin in frames f0 .. f0 + F - 1 (row_origin), 0 without the spread.
 template <int MODE, typename P, int F>
-__device__ __forceinline__ void rows_item(const QueuePlan &qp, int k, int fb, RowsRed &s_red) {
+__device__ __forceinline__ void rows_origin(const QueuePlan &qp, const int4 rec, int f0, double (&o)[F]) {
+    const P *frames = static_cast<const P *>(qp.frames);
+    const int fvalid = MODE == kSpread && is_float_px<P>() ? qp.first_valid[rec.x] : -1;
+#pragma unroll
+    for (int q = 0; q < F; ++q)
+        o[q] = MODE == kSpread
+                   ? double(row_origin<P>(qp.entry_std, rec.w, fvalid, rec.z,
+                                          frames + int64_t(min(f0 + q, qp.n_frames - 1)) * qp.n_pixels))
+                   : 0.0;
+}
+
+// This thread's sums of entries e0 + li, e0 + li + nl, ... < e1 of a row (rec:
+// {row, first entry, end, origin}) in frames f0 .. f0 + F - 1.
+template <int MODE, typename P, int F>
+__device__ __forceinline__ void rows_sum(const QueuePlan &qp, const int4 rec, int e0, int e1, int li,
+                                         int nl, int f0, const double (&o)[F],
+                                         double (&acc)[F][NAcc<MODE, P>::value]) {
     constexpr int NA = NAcc<MODE, P>::value;
     constexpr bool SPREAD = MODE == kSpread;
-    constexpr int NW = kRowsWarps;
-    const int4 *__restrict__ items = qp.item;
-    const int32_t *__restrict__ rows = qp.rows;
-    const int32_t *__restrict__ row_ptr = qp.row_ptr;
     const int2 *__restrict__ entry = qp.entry;
-    const float4 *__restrict__ entry_std = qp.entry_std;
     const float2 *__restrict__ px_norm = qp.px_norm;
-    const int32_t *__restrict__ first_valid = qp.first_valid;
-    const int32_t *__restrict__ origin_entry = qp.origin;
-    const double *__restrict__ den = qp.den;
-    const double *__restrict__ den_std = qp.den_std;
-    const int32_t *__restrict__ valid_std = qp.valid_std;
     const P *__restrict__ frames = static_cast<const P *>(qp.frames);
-    const int64_t n_pixels = qp.n_pixels;
-    const int n_frames = qp.n_frames, n_rows = qp.n_rows;
-    double *__restrict__ out_i = qp.out_i;
-    double *__restrict__ out_s = qp.out_s;
-    double *__restrict__ out_d = qp.out_d;
-    const int4 it = items[k];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // {row, 0, begin, end}: one long row for the whole CTA, its entry range
-    // inline; {first, n > 0}: a row per warp; {first, -n}: tiny rows, 8 lanes
-    // each (four per warp), rows[first ..] and their row pointers.
-    const bool whole = it.y == 0, tiny = it.y < 0;
-    if (!whole && !tiny && warp >= it.y) return;  // no CTA-wide barrier in this case
-    const int sub = int(threadIdx.x) >> 3;
-    if (tiny && (sub & ~3) >= -it.y) return;  // a warp whose four rows are all past the end
-    const bool live = !tiny || sub < -it.y;    // lanes past the end still shuffle
-    const int row = whole ? it.x : rows[it.x + (tiny ? (live ? sub : 0) : warp)];
-    const int e0 = whole ? it.z : row_ptr[row];
-    const int e1 = whole ? it.w : live ? row_ptr[row + 1] : e0;
-    const int li = whole ? int(threadIdx.x) : tiny ? (lane & 7) : lane;
-    const int nl = whole ? kRowsThreads : tiny ? 8 : 32;
-    const int org = SPREAD ? origin_entry[row] : -1, fvalid = SPREAD ? first_valid[row] : -1;
-    // frames [F*fb, F*fb + F) of the batch, one pass
-    for (int f0 = F * fb; f0 < n_frames && f0 < F * fb + F; f0 += F) {
-        const P *fr[F];
+    const P *fr[F];
 #pragma unroll
-        for (int q = 0; q < F; ++q) fr[q] = frames + int64_t(min(f0 + q, n_frames - 1)) * n_pixels;
-        double o[F];
+    for (int q = 0; q < F; ++q)
+        fr[q] = frames + int64_t(min(f0 + q, qp.n_frames - 1)) * qp.n_pixels;
 #pragma unroll
-        for (int q = 0; q < F; ++q)
-            o[q] = SPREAD ? double(row_origin<P>(entry_std, org, fvalid, e1, fr[q])) : 0.0;
-        double acc[F][NA];
+    for (int q = 0; q < F; ++q)
 #pragma unroll
-        for (int q = 0; q < F; ++q)
+        for (int a = 0; a < NA; ++a) acc[q][a] = 0.0;
+    for (int j0 = e0 + li; j0 < e1; j0 += nl * kRowsU) {
+        // Loads past the end repeat the last entry with weight 0 and pixel 0: no
+        // load waits behind a branch.
+        float cw[kRowsU];
+        [[maybe_unused]] float2 nn[kRowsU];
+        P raw[kRowsU][F];
 #pragma unroll
-            for (int a = 0; a < NA; ++a) acc[q][a] = 0.0;
-        for (int j0 = e0 + li; j0 < e1; j0 += nl * kRowsU) {
-            float2 nn[kRowsU];
-            int2 en[kRowsU];
-            double x[kRowsU][F];
+        for (int u = 0; u < kRowsU; ++u) {
+            const int j = j0 + nl * u;
+            const int2 en = entry[min(j, e1 - 1)];
+            const uint32_t col = uint32_t(en.x);
+            cw[u] = j < e1 ? __int_as_float(en.y) : 0.f;
+            if constexpr (SPREAD) nn[u] = px_norm[col];
 #pragma unroll
-            for (int u = 0; u < kRowsU; ++u) {
-                const int j = j0 + nl * u;
-                const bool in = j < e1;
-                en[u] = in ? entry[j] : make_int2(0, 0);
-                const uint32_t col = uint32_t(en[u].x);
-                if constexpr (SPREAD) nn[u] = in ? px_norm[col] : make_float2(0.f, 0.f);
-#pragma unroll
-                for (int q = 0; q < F; ++q) x[u][q] = in ? load_px_d<P>(fr[q], col) : 0.0;
-            }
-#pragma unroll
-            for (int u = 0; u < kRowsU; ++u) {
-                if (j0 + nl * u >= e1) break;
-                if constexpr (SPREAD) {
-                    // valid for the spread (azimuthal.rs:62-75): c > 0 and n
-                    // finite and > 0 ({0, 0} marks an invalid n); an invalid
-                    // entry adds nothing
-                    const float cf = __int_as_float(en[u].y);
-                    const bool ok = nn[u].x > 0.f && cf > 0.f && cf <= 3.40282347e+38f;
-                    const double c = ok ? double(cf) : 0.0;
-                    const double cr = ok ? double(__fdiv_rn(cf, nn[u].x)) : 0.0;
-                    const double n = ok ? __dadd_rn(double(nn[u].x), double(nn[u].y)) : 1.0;
-                    const double c2 = __dmul_rn(c, c);
-#pragma unroll
-                    for (int q = 0; q < F; ++q) {
-                        const double v = x[u][q];
-                        if (is_float_px<P>() && !isfinite(v)) {
-                            acc[q][NA - 2] = __dadd_rn(acc[q][NA - 2], __dmul_rn(c, n));
-                            acc[q][NA - 1] = __dadd_rn(acc[q][NA - 1], c > 0.0 ? 1.0 : 0.0);
-                            continue;
-                        }
-                        acc[q][0] = __fma_rn(c, v, acc[q][0]);
-                        acc[q][1] = __fma_rn(c2, is_unsigned_px<P>() ? v : fmax(v, 0.0), acc[q][1]);
-                        const double t = __fma_rn(-o[q], n, v);
-                        acc[q][2] = __fma_rn(__dmul_rn(cr, t), t, acc[q][2]);
-                        acc[q][kSpreadA] = __fma_rn(c, t, acc[q][kSpreadA]);
-                    }
-                } else {
-                    const double c = __int_as_float(en[u].y);
-                    const double c2 = __dmul_rn(c, c);
-#pragma unroll
-                    for (int q = 0; q < F; ++q) {
-                        acc[q][0] = __fma_rn(c, x[u][q], acc[q][0]);
-                        if (MODE == kErrors)
-                            acc[q][1] = __fma_rn(c2, is_unsigned_px<P>() ? x[u][q] : fmax(x[u][q], 0.0),
-                                                 acc[q][1]);
-                    }
-                }
-            }
+            for (int q = 0; q < F; ++q) raw[u][q] = __ldg(fr[q] + col);
         }
 #pragma unroll
-        for (int q = 0; q < F; ++q)
+        for (int u = 0; u < kRowsU; ++u) {
+            if (is_float_px<P>() && j0 + nl * u >= e1) {
 #pragma unroll
-            for (int a = 0; a < NA; ++a)
-                acc[q][a] = tiny ? group8_sum_d(acc[q][a]) : warp_sum_d(acc[q][a]);
-        if (whole) {
-            if (lane == 0)
+                for (int q = 0; q < F; ++q) raw[u][q] = P(0);
+            }
+            if constexpr (SPREAD) {
+                // valid for the spread (azimuthal.rs:62-75): c > 0 and n
+                // finite and > 0 ({0, 0} marks an invalid n); an invalid
+                // entry adds nothing
+                const float cf = cw[u];
+                const bool ok = nn[u].x > 0.f && cf > 0.f && cf <= 3.40282347e+38f;
+                const double c = ok ? double(cf) : 0.0;
+                const double cr = ok ? double(__fdiv_rn(cf, nn[u].x)) : 0.0;
+                const double n = ok ? __dadd_rn(double(nn[u].x), double(nn[u].y)) : 1.0;
+                const double c2 = __dmul_rn(c, c);
 #pragma unroll
-                for (int q = 0; q < F; ++q)
-#pragma unroll
-                    for (int a = 0; a < NA; ++a) s_red[warp][q * NA + a] = acc[q][a];
-            __syncthreads();
-            if (threadIdx.x == 0)
-#pragma unroll
-                for (int q = 0; q < F; ++q)
-#pragma unroll
-                    for (int a = 0; a < NA; ++a) {
-                        double v = s_red[0][q * NA + a];
-                        for (int w = 1; w < NW; ++w) v = __dadd_rn(v, s_red[w][q * NA + a]);
-                        acc[q][a] = v;
+                for (int q = 0; q < F; ++q) {
+                    const double v = double(raw[u][q]);
+                    if (is_float_px<P>() && !isfinite(v)) {
+                        acc[q][NA - 2] = __dadd_rn(acc[q][NA - 2], __dmul_rn(c, n));
+                        acc[q][NA - 1] = __dadd_rn(acc[q][NA - 1], c > 0.0 ? 1.0 : 0.0);
+                        continue;
                     }
-            __syncthreads();  // s_red is rewritten by the next frames
-            if (threadIdx.x != 0) continue;
-        } else if (tiny ? ((lane & 7) != 0 || !live) : lane != 0) {
-            continue;
-        }
-#pragma unroll
-        for (int q = 0; q < F; ++q) {
-            if (f0 + q >= n_frames) break;
-            const double *v = acc[q];
-            const int64_t oo = int64_t(f0 + q) * n_rows + row;
-            if constexpr (!SPREAD) {
-                const double n = den[row];
-                out_i[oo] = n == 0.0 ? 0.0 : v[0] / n;
-                if (MODE == kErrors) {
-                    const double s2 = n == 0.0 ? 0.0 : v[1] / (n * n);
-                    out_s[oo] = sqrt(s2 > 0.0 ? s2 : 0.0);
+                    acc[q][0] = __fma_rn(c, v, acc[q][0]);
+                    acc[q][1] = __fma_rn(c2, is_unsigned_px<P>() ? v : fmax(v, 0.0), acc[q][1]);
+                    const double t = __fma_rn(-o[q], n, v);
+                    acc[q][2] = __fma_rn(__dmul_rn(cr, t), t, acc[q][2]);
+                    acc[q][kSpreadA] = __fma_rn(c, t, acc[q][kSpreadA]);
                 }
             } else {
-                int valid = valid_std[row];
-                double sw = den_std[row];
-                if (NA == 6) {
-                    valid -= int(v[NA - 1] + 0.5);
-                    sw -= v[NA - 2];
+                const double c = cw[u];
+                const double c2 = __dmul_rn(c, c);
+#pragma unroll
+                for (int q = 0; q < F; ++q) {
+                    const double v = double(raw[u][q]);
+                    acc[q][0] = __fma_rn(c, v, acc[q][0]);
+                    if (MODE == kErrors)
+                        acc[q][1] = __fma_rn(c2, is_unsigned_px<P>() ? v : fmax(v, 0.0), acc[q][1]);
                 }
-                if (valid <= 0 || !(sw > 0.0)) {
-                    out_i[oo] = 0.0;
-                    if (out_s) out_s[oo] = 0.0;
-                    out_d[oo] = __longlong_as_double(0x7ff8000000000000ll);
-                    continue;
-                }
-                const double a1 = v[kSpreadA];
-                out_i[oo] = v[0] / sw;
-                if (out_s) out_s[oo] = sqrt(v[1] > 0.0 ? v[1] : 0.0) / sw;
-                const double mean = a1 / sw;
-                const double q2 = (v[2] - mean * a1) / sw;
-                // one valid contribution: its deviation from itself is exactly 0
-                out_d[oo] = valid == 1 ? 0.0 : sqrt(q2 > 0.0 ? q2 : 0.0);
             }
         }
     }
 }
 
-// Lane mapping 10 for one plan's batch: one CTA per (item, frame block).
-// Resident CTAs per SM the compiler must allow for (0: as many as the
-// registers it chooses leave; the spread's one-frame form takes 64, four CTAs).
-#ifndef DG_ROWS_MINB
-#define DG_ROWS_MINB 0
-#endif
-#if DG_ROWS_MINB > 0
-#define DG_ROWS_BOUNDS __launch_bounds__(kRowsThreads, DG_ROWS_MINB)
-#else
-#define DG_ROWS_BOUNDS __launch_bounds__(kRowsThreads)
-#endif
+// Warp w's eighth of a long row.
+__device__ __forceinline__ int2 rows_eighth(const int4 rec, int w) {
+    const int64_t n = rec.z - rec.y;
+    return make_int2(rec.y + int(n * w / kRowsWarps), rec.y + int(n * (w + 1) / kRowsWarps));
+}
+
+// One row-warp item of a plan's batch (q.item[k]); every thread of the CTA
+// calls it. F frames, one pass over the entries.
 template <int MODE, typename P, int F>
-__global__ void DG_ROWS_BOUNDS k_rows(const QueuePlan q) {
+__device__ __forceinline__ void rows_item(const QueuePlan &qp, int k, int fb, RowsRed &s_red) {
+    constexpr int NA = NAcc<MODE, P>::value;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int f0 = F * fb;  // frames [f0, f0 + F) of the batch
+    double o[F], acc[F][NA];
+    if (k < qp.n_long) {  // a long row for the whole CTA
+        const int4 rec = qp.rows[k];
+        const int2 e = rows_eighth(rec, warp);
+        rows_origin<MODE, P, F>(qp, rec, f0, o);
+        rows_sum<MODE, P, F>(qp, rec, e.x, e.y, lane, 32, f0, o, acc);
+#pragma unroll
+        for (int q = 0; q < F; ++q)
+#pragma unroll
+            for (int a = 0; a < NA; ++a) {
+                acc[q][a] = warp_sum_d(acc[q][a]);
+                if (lane == 0) s_red[warp][q * NA + a] = acc[q][a];
+            }
+        __syncthreads();
+        // the eighths' sums in order, a thread per sum
+        const int t = int(threadIdx.x);
+        if (t < F * NA) {
+            double v = s_red[0][t];
+#pragma unroll
+            for (int w = 1; w < kRowsWarps; ++w) v = __dadd_rn(v, s_red[w][t]);
+            s_red[0][t] = v;
+        }
+        __syncthreads();
+        if (t < F && f0 + t < qp.n_frames) rows_write<MODE, P>(qp, rec.x, f0 + t, &s_red[0][t * NA]);
+        __syncthreads();  // s_red is rewritten by the next item
+        return;
+    }
+    // eight rows, one per warp, or 32 tiny rows, 8 lanes each (four per warp)
+    const bool tiny = k >= qp.n_long + qp.n_mid;
+    const int first = tiny ? qp.first_tiny + (k - qp.n_long - qp.n_mid) * 4 * kRowsWarps
+                           : qp.n_long + (k - qp.n_long) * kRowsWarps;
+    const int end = tiny ? qp.n_rows : qp.first_tiny;
+    const int at = first + (tiny ? int(threadIdx.x) >> 3 : warp);
+    if ((tiny ? first + 4 * warp : at) >= end) return;  // a warp whose rows are all past the end
+    const bool live = at < end;                         // lanes past the end still shuffle
+    const int4 rec = qp.rows[live ? at : first];
+    const int li = tiny ? lane & 7 : lane;
+    rows_origin<MODE, P, F>(qp, rec, f0, o);
+    rows_sum<MODE, P, F>(qp, rec, rec.y, live ? rec.z : rec.y, li, tiny ? 8 : 32, f0, o, acc);
+#pragma unroll
+    for (int q = 0; q < F; ++q)
+#pragma unroll
+        for (int a = 0; a < NA; ++a)
+            acc[q][a] = tiny ? group8_sum_d(acc[q][a]) : warp_sum_d(acc[q][a]);
+    if (li == 0 && live) {
+#pragma unroll
+        for (int q = 0; q < F; ++q)
+            if (f0 + q < qp.n_frames) rows_write<MODE, P>(qp, rec.x, f0 + q, acc[q]);
+    }
+}
+
+// Eight neighbouring long rows, a warp each, which walks its row's eighths one
+// after the other: the warps read the same pixels about the same time and share
+// their sectors in L1. The sums are those of rows_item, bit for bit.
+template <int MODE, typename P, int F>
+__device__ __forceinline__ void rows_group(const QueuePlan &qp, int group, int fb, RowsRed &s_red) {
+    constexpr int NA = NAcc<MODE, P>::value;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = group * kRowsWarps + warp;
+    if (k >= qp.n_long) return;
+    const int4 rec = qp.rows[k];
+    const int f0 = F * fb;
+    double o[F], acc[F][NA];
+    rows_origin<MODE, P, F>(qp, rec, f0, o);
+    for (int w = 0; w < kRowsWarps; ++w) {
+        const int2 e = rows_eighth(rec, w);
+        rows_sum<MODE, P, F>(qp, rec, e.x, e.y, lane, 32, f0, o, acc);
+#pragma unroll
+        for (int q = 0; q < F; ++q)
+#pragma unroll
+            for (int a = 0; a < NA; ++a) {
+                acc[q][a] = warp_sum_d(acc[q][a]);
+                if (lane == 0) {
+                    double &v = s_red[warp][q * NA + a];
+                    v = w == 0 ? acc[q][a] : __dadd_rn(v, acc[q][a]);
+                }
+            }
+    }
+    __syncwarp();
+    if (lane < F && f0 + lane < qp.n_frames)
+        rows_write<MODE, P>(qp, rec.x, f0 + lane, &s_red[warp][lane * NA]);
+}
+
+// The rows' origin entries beside their ranges, so that a launch reads one record
+// a row.
+__global__ void k_row_origins(int4 *__restrict__ rows, const int32_t *__restrict__ origin, int n) {
+    const int i = int(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i < n) rows[i].w = origin[rows[i].x];
+}
+
+// Lane mapping 10 for one plan's batch: one CTA per (item, frame block).
+// Resident CTAs per SM the compiler must allow for: what hides the loads' latency
+// is warps. One frame without the spread, 8 (32 registers) against 6: Eiger-4M cake
+// 59.4 and 67.6 us; the others 4 (64 registers) against what the compiler takes:
+// two frames with the spread 69.6 and 75.9, 64 Eiger-9M frames 708 and 738. Four
+// frames with the spread would spill (186 against 125). A launch that leaves SMs
+// with few CTAs anyway (small, one frame) takes the registers that shorten it.
+template <int MODE>
+constexpr int rows_min_ctas(int f, bool small) {
+    return small ? 1 : MODE != kSpread ? (f == 1 ? 8 : 4) : f == 4 ? 1 : 4;
+}
+template <int MODE, typename P, int F, bool SMALL = false>
+__global__ void __launch_bounds__(kRowsThreads, rows_min_ctas<MODE>(F, SMALL)) k_rows(const QueuePlan q, const int groups) {
     __shared__ RowsRed s_red;
-    rows_item<MODE, P, F>(q, blockIdx.x, blockIdx.y, s_red);
+    int k = blockIdx.x;
+    if constexpr (F == 4) {
+        if (k < groups) return rows_group<MODE, P, F>(q, k, blockIdx.y, s_red);
+        if (groups) k += q.n_long - groups;
+    }
+    rows_item<MODE, P, F>(q, k, blockIdx.y, s_red);
 }
 
 // Frames per pass (and per frame block) of a row-warp launch of nf frames.
@@ -1564,11 +1636,23 @@ template <int MODE, typename P>
 void launch_rows(const GatherTable &t, const P *fp, int64_t n_pixels, int nf, double *oi,
                  double *os, double *od, cudaStream_t s) {
     const QueuePlan q = queue_plan(t, fp, n_pixels, nf, oi, os, od);
-    const dim3 grid(unsigned(q.n_items), unsigned(q.frame_blocks));
+    // Long rows in groups of eight (rows_group) once those fill the chip: a group is
+    // a serial walk of eight rows. Eiger-4M with the spread, 235 groups, us, a CTA
+    // per row against groups: 4 frames 122 / 170, 16 frames 442 / 352, 64 frames 1721
+    // / 1347; Eiger-9M intensities, 124 groups: 8 frames 93 / 166, 16 frames 182 /
+    // 190, 32 frames 358 / 337, 64 frames 709 / 596. Four per SM is where they cross.
+    int groups = (q.n_long + kRowsWarps - 1) / kRowsWarps;
+    if (rows_pass_frames(nf) < 4 || int64_t(groups) * q.frame_blocks < 4 * sm_count()) groups = 0;
+    const dim3 grid(unsigned(q.n_items - (groups ? q.n_long - groups : 0)), unsigned(q.frame_blocks));
     switch (rows_pass_frames(nf)) {
-    case 1: k_rows<MODE, P, 1><<<grid, kRowsThreads, 0, s>>>(q); break;
-    case 2: k_rows<MODE, P, 2><<<grid, kRowsThreads, 0, s>>>(q); break;
-    default: k_rows<MODE, P, 4><<<grid, kRowsThreads, 0, s>>>(q); break;
+    case 1:
+        if (q.n_items <= 2 * sm_count())
+            k_rows<MODE, P, 1, true><<<grid, kRowsThreads, 0, s>>>(q, groups);
+        else
+            k_rows<MODE, P, 1><<<grid, kRowsThreads, 0, s>>>(q, groups);
+        break;
+    case 2: k_rows<MODE, P, 2><<<grid, kRowsThreads, 0, s>>>(q, groups); break;
+    default: k_rows<MODE, P, 4><<<grid, kRowsThreads, 0, s>>>(q, groups); break;
     }
     DG_CUDA(cudaGetLastError());
 }
@@ -1887,44 +1971,41 @@ void make_gather_table(const DeviceCsr &table, const double *d_norm, int32_t dim
     }
     DG_CUDA(cudaMemcpyAsync(out.row_seg.ptr, row_seg.data(), row_seg.size() * 4,
                             cudaMemcpyHostToDevice, s));
-    // Row warps (mapping 10): long rows one per CTA, longest first; the
-    // others eight per CTA in row order.
-    std::vector<int32_t> rw_ptr, rw_rows;
-    std::vector<int4> rw_items;
+    // Row warps (mapping 10): long rows one to a CTA, longest first;
+    // the others eight or 32 per CTA in row order.
+    std::vector<int4> rw_rows;
     if (table.nnz <= INT32_MAX && nb > 0) {
-        rw_ptr.assign(rp.begin(), rp.end());
-        for (int64_t r = 0; r < nb; ++r)
-            if (rp[size_t(r) + 1] - rp[size_t(r)] > kRowsLong) rw_rows.push_back(int32_t(r));
-        std::stable_sort(rw_rows.begin(), rw_rows.end(), [&](int32_t a, int32_t b) {
-            return rp[size_t(a) + 1] - rp[size_t(a)] > rp[size_t(b) + 1] - rp[size_t(b)];
-        });
-        for (size_t i = 0; i < rw_rows.size(); ++i) {  // long rows carry their range
-            const int32_t r = rw_rows[i];
-            rw_items.push_back(make_int4(r, 0, int(rp[size_t(r)]), int(rp[size_t(r) + 1])));
-        }
         auto len = [&](int64_t r) { return rp[size_t(r) + 1] - rp[size_t(r)]; };
-        const size_t first_mid = rw_rows.size();
-        for (int64_t r = 0; r < nb; ++r)
-            if (len(r) <= kRowsLong && len(r) > kRowsTiny) rw_rows.push_back(int32_t(r));
-        for (size_t i = first_mid; i < rw_rows.size(); i += kRowsWarps)
-            rw_items.push_back(make_int4(int(i), int(std::min<size_t>(kRowsWarps,
-                                                                      rw_rows.size() - i)), 0, 0));
-        const size_t first_tiny = rw_rows.size();
-        for (int64_t r = 0; r < nb; ++r)
-            if (len(r) <= kRowsTiny) rw_rows.push_back(int32_t(r));
-        for (size_t i = first_tiny; i < rw_rows.size(); i += 4 * kRowsWarps)
-            rw_items.push_back(make_int4(int(i), -int(std::min<size_t>(4 * kRowsWarps,
-                                                                       rw_rows.size() - i)), 0, 0));
-        out.rw_row_ptr.alloc(rw_ptr.size());
+        auto take = [&](int64_t above, int64_t most) {  // rows of above < entries <= most
+            for (int64_t r = 0; r < nb; ++r)
+                if (len(r) > above && len(r) <= most)
+                    rw_rows.push_back(make_int4(int(r), int(rp[size_t(r)]), int(rp[size_t(r) + 1]), -1));
+            return int32_t(rw_rows.size());
+        };
+        out.rw_long = take(kRowsLong, INT64_MAX);
+        // neighbours stay together in groups of kRowsWarps, the longest rows first
+        std::vector<int4> by_row(rw_rows);
+        std::vector<std::pair<int64_t, size_t>> groups;
+        for (size_t i = 0; i < by_row.size(); i += kRowsWarps) {
+            int64_t n = 0;
+            for (size_t j = i; j < std::min(by_row.size(), i + kRowsWarps); ++j) n += len(by_row[j].x);
+            groups.push_back({by_row.size() - i < size_t(kRowsWarps) ? 0 : -n, i});
+        }
+        std::stable_sort(groups.begin(), groups.end());  // a group of fewer comes last
+        rw_rows.clear();
+        for (const auto &g : groups)
+            for (size_t j = g.second; j < std::min(by_row.size(), g.second + kRowsWarps); ++j)
+                rw_rows.push_back(by_row[j]);
+        out.rw_tiny = take(kRowsTiny, kRowsLong);
+        take(-1, kRowsTiny);
+        out.rw_n_items = out.rw_long + (out.rw_tiny - out.rw_long + kRowsWarps - 1) / kRowsWarps +
+                         int32_t((nb - out.rw_tiny + 4 * kRowsWarps - 1) / (4 * kRowsWarps));
         out.rw_rows.alloc(rw_rows.size());
-        out.rw_item.alloc(rw_items.size());
-        DG_CUDA(cudaMemcpyAsync(out.rw_row_ptr.ptr, rw_ptr.data(), rw_ptr.size() * 4,
+        DG_CUDA(cudaMemcpyAsync(out.rw_rows.ptr, rw_rows.data(), rw_rows.size() * sizeof(int4),
                                 cudaMemcpyHostToDevice, s));
-        DG_CUDA(cudaMemcpyAsync(out.rw_rows.ptr, rw_rows.data(), rw_rows.size() * 4,
-                                cudaMemcpyHostToDevice, s));
-        DG_CUDA(cudaMemcpyAsync(out.rw_item.ptr, rw_items.data(), rw_items.size() * sizeof(int4),
-                                cudaMemcpyHostToDevice, s));
-        out.rw_n_items = int32_t(rw_items.size());
+        k_row_origins<<<unsigned((nb + 255) / 256), 256, 0, s>>>(out.rw_rows.ptr, out.origin.ptr,
+                                                                 int(nb));
+        DG_CUDA(cudaGetLastError());
     }
     DG_CUDA(cudaStreamSynchronize(s));
     out.strip_first = std::move(strip_first);
@@ -1986,15 +2067,12 @@ void reserve_partials(GatherTable &t, int64_t n_frames, uint32_t flags, int dtyp
 QueuePlan queue_plan(const GatherTable &t, const void *d_frames, int64_t n_pixels, int n_frames,
                      double *oi, double *os, double *od) {
     QueuePlan q{};
-    q.item = t.rw_item.ptr;
     q.rows = t.rw_rows.ptr;
-    q.row_ptr = t.rw_row_ptr.ptr;
     q.entry = t.entry.ptr;
     q.entry_std = t.entry_std.ptr;
     q.entry_nlo = t.entry_nlo.ptr;
     q.px_norm = t.px_norm.ptr;
     q.first_valid = t.first_valid.ptr;
-    q.origin = t.origin.ptr;
     q.den = t.den.ptr;
     q.den_std = t.den_std.ptr;
     q.valid_std = t.valid_std.ptr;
@@ -2006,6 +2084,9 @@ QueuePlan queue_plan(const GatherTable &t, const void *d_frames, int64_t n_pixel
     q.n_frames = n_frames;
     q.n_rows = t.n_rows;
     q.n_items = n_frames > 0 ? t.rw_n_items : 0;
+    q.n_long = t.rw_long;
+    q.n_mid = (t.rw_tiny - t.rw_long + kRowsWarps - 1) / kRowsWarps;
+    q.first_tiny = t.rw_tiny;
     q.frame_blocks = std::max(1, (n_frames + rows_pass_frames(n_frames) - 1) /
                                      rows_pass_frames(n_frames));
     return q;

@@ -325,19 +325,17 @@ struct GatherTable {
     DeviceArray<uint64_t> mask_words;  // scratch: per-frame masks as words (bin tiles)
     // Bin tiles (k_gather_bins), mappings 7 and 8; see dg_gather.cu.
     BinTiles bt[2];
-    // Row warps (k_rows), mapping 10: row pointers, rows with more than
-    // kRowsLong entries (longest first) then the others, and one item per
-    // CTA: {row, 0, entry begin, entry end} for a long row, {first in
-    // rw_rows, count <= 8} for rows taken one per warp, {first, -count <= 32}
-    // for rows of at most kRowsTiny entries taken eight lanes each.
+    // Row warps (k_rows), mapping 10: per row {row, entry begin, entry end, origin
+    // entry}: rw_long rows of more than kRowsLong entries, longest first (a CTA
+    // each), then to rw_tiny the rows of more than kRowsTiny (eight per CTA, a warp
+    // each), then the others (32 per CTA, eight lanes each); rw_n_items CTAs.
+    int32_t rw_long = 0, rw_tiny = 0;
     int32_t rw_n_items = 0;
     // Per pixel (frame storage order) its norm n as an FP32 pair {n, n - n32},
     // {0, 0} where n is not finite or not positive: the row warps' spread
     // reads the 8-byte entries and gathers n beside the pixel.
     DeviceArray<float2> px_norm;
-    DeviceArray<int32_t> rw_row_ptr;
-    DeviceArray<int32_t> rw_rows;
-    DeviceArray<int4> rw_item;
+    DeviceArray<int4> rw_rows;
     int variant = 0;                  // gather lane mapping (dg_gather.cu kVariantCount)
     int withhold_test = 0;            // bin tiles: stall one warp (dg_plan_test_wait_timeout)
     int32_t flip_rows = 0, flip_cols = 0;  // frames stored bottom row first (0: detector order)
@@ -398,15 +396,12 @@ void reserve_partials(GatherTable &t, int64_t n_frames, uint32_t flags, int dtyp
 // until total_items are done; item_first is the prefix index of a plan's
 // first tile.
 struct QueuePlan {
-    const int4 *item;
-    const int32_t *rows;
-    const int32_t *row_ptr;
+    const int4 *rows;      // {row, first entry, end, origin}
     const int2 *entry;
     const float4 *entry_std;
     const float *entry_nlo;
     const float2 *px_norm;
     const int32_t *first_valid;
-    const int32_t *origin;
     const double *den;
     const double *den_std;
     const int32_t *valid_std;
@@ -417,7 +412,7 @@ struct QueuePlan {
     int32_t n_items;       // row items
     int32_t frame_blocks;  // blocks of up to four frames (one pass each)
     int32_t item_first;    // the work queue: first (item, frame block) tile
-    int32_t pad;
+    int32_t n_long, n_mid, first_tiny;  // CTAs of long and of mid rows; the first tiny row
 };
 struct QueueHeader {
     int32_t n_plans, total_items, counter, pad;  // counter: 0 before each launch
