@@ -169,7 +169,8 @@ DG_EXPORT dg_status dg_integrate_device(dg_plan *plan, const void *d_frames, int
  * no cudaMalloc or cudaFree; the plan (from dg_plan_create, which does
  * allocate) and the frames and results are the caller's. A plan whose partial
  * sums for a single frame exceed the array is rejected with
- * DG_UNSUPPORTED. The first call on a device looks up the array's device
+ * DG_UNSUPPORTED (row warps keep none, bin tiles some 0.2 MiB per frame for the
+ * tiles they cut). The first call on a device looks up the array's device
  * address (cudaGetSymbolAddress); make it before any stream capture. All
  * calls on a device share the array, so calls that overlap on the GPU race:
  * serialise them. Results equal dg_integrate_device's. */
