@@ -497,6 +497,31 @@ dg_status dg_plan_test_wait_timeout(dg_plan *plan, const void *d_frames, int32_t
     });
 }
 
+dg_status dg_test_bin_items(int32_t variant, int64_t n_rows, const int64_t *row_ptr,
+                            const int32_t *col, int64_t counts[4], int32_t *items,
+                            int64_t *first_chunk, int32_t *spans, int32_t *row_part,
+                            int32_t *part_ids) {
+    return guarded([&] {
+        if (!row_ptr || !col || !counts || n_rows < 1)
+            dg::fail(DG_INVALID_INPUT, "a table of at least one row and counts are needed");
+        dg::BinItems b;
+        dg::bin_items(variant, n_rows, row_ptr, col, b);
+        counts[0] = int64_t(b.items.size());
+        counts[1] = b.rows;
+        counts[2] = int64_t(b.first_chunk.size()) - 1;
+        counts[3] = int64_t(b.part_ids.size());
+        auto put = [](const auto &v, auto *out) {
+            if (out && !v.empty()) std::memcpy(out, v.data(), v.size() * sizeof v[0]);
+        };
+        put(b.items, items);
+        put(b.first_chunk, first_chunk);
+        put(b.spans[0], spans);
+        put(b.spans[1], spans ? spans + 4 * b.spans[0].size() : nullptr);
+        put(b.row_part, row_part);
+        put(b.part_ids, part_ids);
+    });
+}
+
 namespace {
 
 // Arguments of the per-frame-mask and raw-sum calls.

@@ -78,7 +78,8 @@ constexpr int kBtFoldPairs = 32;
 constexpr int kBtPieceMin = 64, kBtPieceMax = 96;
 
 // Claimed items in flight between the claiming warp and the other producers: a
-// producer is at most BUFS chunks, so at most BUFS + 1 items, behind it.
+// producer is at most BUFS chunks, so at most BUFS + 1 items (every item has a
+// chunk), behind it.
 constexpr int kBtWork = 8;
 
 // One bin-tile layout: rows per tile (= consumer warps), chunk capacities,
@@ -986,58 +987,77 @@ __global__ void __launch_bounds__(256)
 
 }  // namespace
 
+// A tile on the host: runs of chunks, pixels and pairs are relative to it.
+struct BinTile {
+    std::vector<int4> chunks;      // {px offset, D, pair offset, pairs}
+    std::vector<int32_t> cpair;    // per chunk kRows + 1
+    std::vector<int32_t> px;
+    std::vector<int4> pairs;       // {slot0, slot1, entry0, entry1}
+    int64_t entries = 0;
+};
+// A piece of a tile: its chunks and, where the tile is cut, per fold cadence and
+// row the {chunk, pair} to start and to end at, chunks relative to c0.
+struct BinPiece {
+    int64_t tile;
+    int c0, n;
+    std::vector<int4> spans[2];
+};
+// The tiles of a table and their pieces (items) in claim order.
+struct BinLayout {
+    std::vector<BinTile> tiles;
+    std::vector<std::vector<BinPiece>> cut;
+    std::vector<int64_t> first_chunk;         // per tile, then the number of chunks
+    std::vector<int4> items;                  // {first row, rows, first chunk, chunks}
+    bool split = false;                       // with the lists below
+    std::vector<int4> spans[2];               // per item and row
+    std::vector<int32_t> row_part, part_ids;  // every row's pieces (item * kRows + row), in order
+};
+
+// fn(0) .. fn(count - 1) over host threads.
+template <class Fn>
+void parallel(int64_t count, Fn &&fn) {
+    const int nt = int(std::min<int64_t>(
+        count, std::max(1u, std::min(16u, std::thread::hardware_concurrency()))));
+    std::vector<std::thread> pool;
+    std::atomic<int64_t> next{0};
+    for (int t = 0; t < nt; ++t)
+        pool.emplace_back([&]() {
+            for (int64_t i; (i = next.fetch_add(1)) < count;) fn(i);
+        });
+    for (auto &th : pool) th.join();
+}
+
 // Bin tiles (k_gather_bins) at plan time, on the host: for every run of
 // CFG::kRows rows, the rows' entries merged in pixel order and cut into chunks of
 // at most kBtDCap distinct pixels and kBtPCap pairs (a new pixel that would
 // exceed either opens the next chunk, so a chunk is a pixel-index interval
 // and each row's entries in it are a contiguous run of its CSR row). Tiles
-// are cut into pieces (see the file comment). Each row keeps {origin entry,
-// first valid entry, row end} for the spread's origin (row_origin), read before
-// the first chunk. A chunk's first pair is even, so
+// are cut into pieces (see the file comment). A chunk's first pair is even, so
 // that its pairs C are copied from a 16-byte boundary.
 template <class CFG>
-void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cudaStream_t s) {
+void lay_out_bin_tiles(const int64_t *rp, const int32_t *col, int64_t nb, BinLayout &out) {
     constexpr int kBtDCap = CFG::kDCap, kBtPCap = CFG::kPCap, kBtRows = CFG::kRows;
-    constexpr int kBtMetaHead = CFG::kMetaHead, kBtMetaWords = CFG::kMetaWords;
-    const int64_t nb = table.n_rows;
-    out.n_items = 0;
-    if (nb == 0 || table.nnz == 0) return;
-    out.wait_err.alloc();
-    std::vector<int64_t> rp(static_cast<size_t>(nb) + 1);
-    DG_CUDA(cudaMemcpyAsync(rp.data(), table.row_ptr.ptr, rp.size() * 8, cudaMemcpyDeviceToHost, s));
-    std::vector<int32_t> col(static_cast<size_t>(table.nnz)), fv(static_cast<size_t>(nb)),
-        oe(static_cast<size_t>(nb));
-    DG_CUDA(cudaMemcpyAsync(col.data(), table.col.ptr, col.size() * 4, cudaMemcpyDeviceToHost, s));
-    DG_CUDA(cudaMemcpyAsync(fv.data(), gt.first_valid.ptr, fv.size() * 4, cudaMemcpyDeviceToHost, s));
-    DG_CUDA(cudaMemcpyAsync(oe.data(), gt.origin.ptr, oe.size() * 4, cudaMemcpyDeviceToHost, s));
-    DG_CUDA(cudaStreamSynchronize(s));
     const int64_t n_items = (nb + kBtRows - 1) / kBtRows;
-    struct Tile {
-        std::vector<int4> chunks;      // {px offset, D, pair offset, pairs} (tile-relative)
-        std::vector<int32_t> cpair;    // per chunk kBtRows + 1
-        std::vector<int32_t> px;
-        std::vector<int4> pairs;       // {slot0, slot1, entry0, entry1}
-        int64_t entries = 0;
-    };
-    std::vector<Tile> tiles(static_cast<size_t>(n_items));
+    std::vector<BinTile> &tiles = out.tiles;
+    tiles.resize(static_cast<size_t>(n_items));
     auto build = [&](int64_t ti) {
-        Tile &T = tiles[size_t(ti)];
+        BinTile &T = tiles[size_t(ti)];
         const int64_t r0 = ti * kBtRows, r1 = std::min<int64_t>(nb, r0 + kBtRows);
         const int nr = int(r1 - r0);
         // Entries merged in pixel order, rows ascending within a pixel: keys
         // pixel << 32 | row << 27 | position in row; each row is sorted
         // already, so four rounds of pairwise merges order the tile.
-        const int64_t n_e = rp[size_t(r1)] - rp[size_t(r0)];
+        const int64_t n_e = rp[r1] - rp[r0];
         std::vector<uint64_t> ka(static_cast<size_t>(n_e)), kb(static_cast<size_t>(n_e));
         std::vector<int64_t> bounds(static_cast<size_t>(kBtRows) + 1, 0);
         for (int j = 0; j < nr; ++j) {
-            const int64_t b = rp[size_t(r0 + j)], e = rp[size_t(r0 + j) + 1];
+            const int64_t b = rp[r0 + j], e = rp[r0 + j + 1];
             if (e - b >= (int64_t(1) << 27)) fail(DG_UNSUPPORTED, "a bin too large for bin tiles");
-            uint64_t *o = ka.data() + (b - rp[size_t(r0)]);
+            uint64_t *o = ka.data() + (b - rp[r0]);
             for (int64_t k = b; k < e; ++k)
-                o[k - b] = (uint64_t(uint32_t(col[size_t(k)])) << 32) | (uint64_t(j) << 27) |
+                o[k - b] = (uint64_t(uint32_t(col[k])) << 32) | (uint64_t(j) << 27) |
                            uint64_t(k - b);
-            bounds[size_t(j) + 1] = e - rp[size_t(r0)];
+            bounds[size_t(j) + 1] = e - rp[r0];
         }
         for (int j = nr; j < kBtRows; ++j) bounds[size_t(j) + 1] = n_e;
         for (int width = 1; width < kBtRows; width *= 2) {
@@ -1056,7 +1076,7 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
         for (int64_t i = 0; i < n_e; ++i) {
             const uint64_t key = ka[size_t(i)];
             const int j = int((key >> 27) & 31u);
-            m[size_t(i)] = {int32_t(key >> 32), j, int32_t(rp[size_t(r0 + j)] + int64_t(key & ((1u << 27) - 1)))};
+            m[size_t(i)] = {int32_t(key >> 32), j, int32_t(rp[r0 + j] + int64_t(key & ((1u << 27) - 1)))};
         }
         T.entries = n_e;
         T.pairs.reserve(size_t(n_e / 2 + 64));
@@ -1116,24 +1136,13 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
             T.pairs.assign(2, make_int4(kBtDCap, kBtDCap, -1, -1));
         }
     };
-    const int nt = int(std::min<int64_t>(
-        n_items, std::max(1u, std::min(16u, std::thread::hardware_concurrency()))));
-    auto parallel = [&](auto &&fn, int64_t count) {
-        std::vector<std::thread> pool;
-        std::atomic<int64_t> next{0};
-        for (int t = 0; t < nt; ++t)
-            pool.emplace_back([&]() {
-                for (int64_t i; (i = next.fetch_add(1)) < count;) fn(i);
-            });
-        for (auto &th : pool) th.join();
-    };
-    parallel(build, n_items);
+    parallel(n_items, build);
     // Pieces: a tile of many chunks is cut at chunk boundaries, each row at the
     // first fold of its FP32 sums at or after the cut (spans). Both fold
     // cadences (steps of kU2 pairs, and of two for float pixels with the
     // spread) get their own spans; a piece's chunks cover both.
     int64_t all_chunks = 0;
-    for (const Tile &T : tiles) all_chunks += int64_t(T.chunks.size());
+    for (const BinTile &T : tiles) all_chunks += int64_t(T.chunks.size());
     const int piece = int(std::clamp<int64_t>(all_chunks / 350, kBtPieceMin, kBtPieceMax));
     // Neighbouring tiles whose pieces are claimed one after the other: they walk the
     // same rows at the same time and share the sectors at their common edges (Eiger-4M
@@ -1141,15 +1150,11 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
     // tiles 1749). Frames of few pieces need an even finish more (Pilatus 1M, 50 frames:
     // 2 tiles 109 us, 4 tiles 113, 5 tiles 129; 256 frames: 405, 412, 410).
     const int64_t near = piece == kBtPieceMax ? 4 : 2;
-    struct Piece {
-        int64_t tile;
-        int c0, n;                      // chunks of the tile
-        std::vector<int4> spans[2];     // per row, relative to c0
-    };
-    std::vector<std::vector<Piece>> cut(static_cast<size_t>(n_items));
+    std::vector<std::vector<BinPiece>> &cut = out.cut;
+    cut.resize(static_cast<size_t>(n_items));
     std::atomic<bool> any_cut{false};
     auto split = [&](int64_t ti) {
-        const Tile &T = tiles[size_t(ti)];
+        const BinTile &T = tiles[size_t(ti)];
         const int nch = int(T.chunks.size());
         std::vector<int> at;  // first chunk of every piece
         int most = 0;  // neighbouring tiles are cut alike
@@ -1159,7 +1164,7 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
         for (int q = 0; q < parts; ++q) at.push_back(int(int64_t(nch) * q / parts));
         const int k = int(at.size());
         at.push_back(nch);
-        std::vector<Piece> &out_p = cut[size_t(ti)];
+        std::vector<BinPiece> &out_p = cut[size_t(ti)];
         out_p.resize(size_t(k));
         for (int i = 0; i < k; ++i) {
             out_p[size_t(i)].tile = ti;
@@ -1167,7 +1172,6 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
             out_p[size_t(i)].n = at[size_t(i) + 1] - at[size_t(i)];
         }
         if (k == 1) return;
-        any_cut = true;
         const int nr = int(std::min<int64_t>(nb, (ti + 1) * kBtRows) - ti * kBtRows);
         // start[cadence][piece][row]: {chunk, pair of the row's run in it}
         std::vector<std::pair<int, int>> start[2];
@@ -1208,7 +1212,7 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
                     lo = std::min(lo, a.first);
                     hi = std::max(hi, e.second > 0 ? e.first + 1 : e.first);
                 }
-            Piece &p = out_p[size_t(i)];
+            BinPiece &p = out_p[size_t(i)];
             p.c0 = std::min(lo, hi);
             p.n = hi - p.c0;
             for (int s2 = 0; s2 < 2; ++s2) {
@@ -1221,23 +1225,32 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
                 }
             }
         }
+        // A piece in which no row folds holds nothing (a small tile cut like its
+        // large neighbour): its neighbours' spans meet, and no warp would see it.
+        out_p.erase(std::remove_if(out_p.begin(), out_p.end(), [](const BinPiece &p) { return p.n == 0; }),
+                    out_p.end());
+        if (out_p.size() > 1) {
+            any_cut = true;
+            return;
+        }
+        out_p.assign(1, {ti, 0, nch, {}});
     };
-    parallel(split, n_items);
-    std::vector<Piece *> order;
+    parallel(n_items, split);
+    std::vector<const BinPiece *> order;
     for (auto &v : cut)
-        for (Piece &p : v) order.push_back(&p);
+        for (const BinPiece &p : v) order.push_back(&p);
     if (any_cut)  // largest first; whole tiles in tile order
     {
         // largest first, the pieces of neighbouring tiles side by side
         std::map<std::pair<int64_t, int>, int> size;
-        auto key = [&](const Piece *p) {
+        auto key = [&](const BinPiece *p) {
             return std::make_pair(p->tile / near, int(p - cut[size_t(p->tile)].data()));
         };
-        for (const Piece *p : order) {
+        for (const BinPiece *p : order) {
             int &n = size[key(p)];
             n = std::max(n, p->n);
         }
-        std::stable_sort(order.begin(), order.end(), [&](const Piece *a, const Piece *b) {
+        std::stable_sort(order.begin(), order.end(), [&](const BinPiece *a, const BinPiece *b) {
             const auto ka = key(a), kb = key(b);
             const int na = size[ka], nb2 = size[kb];
             if (na != nb2) return na > nb2;
@@ -1246,13 +1259,70 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
         });
     }
     out.split = any_cut;
+    out.first_chunk.assign(size_t(n_items) + 1, 0);
+    for (int64_t i = 0; i < n_items; ++i)
+        out.first_chunk[size_t(i) + 1] = out.first_chunk[size_t(i)] + int64_t(tiles[size_t(i)].chunks.size());
+    if (out.first_chunk.back() > INT32_MAX) fail(DG_UNSUPPORTED, "table too large for bin tiles");
+    out.items.resize(order.size());
+    for (size_t i = 0; i < order.size(); ++i) {
+        const BinPiece &p = *order[i];
+        if (p.n < 1) fail(DG_DEVICE, "a bin-tile item without chunks");
+        const int64_t r0 = p.tile * kBtRows;
+        out.items[i] = make_int4(int(r0), int(std::min<int64_t>(nb, r0 + kBtRows) - r0),
+                                 int(out.first_chunk[size_t(p.tile)]) + p.c0, p.n);
+    }
+    if (!out.split) return;
+    // Spans per item and row, and the pieces of every row in tile order
+    // (partial sums are kept per item and row).
+    std::vector<std::vector<int32_t>> slot(static_cast<size_t>(n_items));
+    for (int64_t ti = 0; ti < n_items; ++ti) slot[size_t(ti)].resize(cut[size_t(ti)].size());
+    for (size_t i = 0; i < order.size(); ++i) {
+        const BinPiece &p = *order[i];
+        slot[size_t(p.tile)][size_t(order[i] - cut[size_t(p.tile)].data())] = int32_t(i);
+        for (int s2 = 0; s2 < 2; ++s2) {
+            if (p.spans[s2].empty())  // an uncut tile
+                out.spans[s2].insert(out.spans[s2].end(), size_t(kBtRows), make_int4(0, 0, INT_MAX, 0));
+            else
+                out.spans[s2].insert(out.spans[s2].end(), p.spans[s2].begin(), p.spans[s2].end());
+        }
+    }
+    out.row_part.assign(size_t(nb) + 1, 0);
+    for (int64_t r = 0; r < nb; ++r) {
+        for (int32_t i : slot[size_t(r / kBtRows)])
+            out.part_ids.push_back(i * kBtRows + int32_t(r % kBtRows));
+        out.row_part[size_t(r) + 1] = int32_t(out.part_ids.size());
+    }
+}
+
+// The bin tiles of a plan's table in device memory. Each row keeps {origin entry,
+// first valid entry, row end} for the spread's origin (row_origin), read before
+// the first chunk.
+template <class CFG>
+void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cudaStream_t s) {
+    constexpr int kBtRows = CFG::kRows;
+    constexpr int kBtMetaHead = CFG::kMetaHead, kBtMetaWords = CFG::kMetaWords;
+    const int64_t nb = table.n_rows;
+    out.n_items = 0;
+    if (nb == 0 || table.nnz == 0) return;
+    out.wait_err.alloc();
+    std::vector<int64_t> rp(static_cast<size_t>(nb) + 1);
+    DG_CUDA(cudaMemcpyAsync(rp.data(), table.row_ptr.ptr, rp.size() * 8, cudaMemcpyDeviceToHost, s));
+    std::vector<int32_t> col(static_cast<size_t>(table.nnz)), fv(static_cast<size_t>(nb)),
+        oe(static_cast<size_t>(nb));
+    DG_CUDA(cudaMemcpyAsync(col.data(), table.col.ptr, col.size() * 4, cudaMemcpyDeviceToHost, s));
+    DG_CUDA(cudaMemcpyAsync(fv.data(), gt.first_valid.ptr, fv.size() * 4, cudaMemcpyDeviceToHost, s));
+    DG_CUDA(cudaMemcpyAsync(oe.data(), gt.origin.ptr, oe.size() * 4, cudaMemcpyDeviceToHost, s));
+    DG_CUDA(cudaStreamSynchronize(s));
+    BinLayout layout;
+    lay_out_bin_tiles<CFG>(rp.data(), col.data(), nb, layout);
+    std::vector<BinTile> &tiles = layout.tiles;
+    out.split = layout.split;
     // Output offsets of every tile, then the tiles copied in parallel.
-    const int64_t n_slots = n_items;
-    std::vector<int64_t> o_ch(size_t(n_slots) + 1, 0), o_px(size_t(n_slots) + 1, 0),
-        o_pr(size_t(n_slots) + 1, 0);
+    const int64_t n_slots = int64_t(tiles.size());
+    const std::vector<int64_t> &o_ch = layout.first_chunk;
+    std::vector<int64_t> o_px(size_t(n_slots) + 1, 0), o_pr(size_t(n_slots) + 1, 0);
     for (int64_t i = 0; i < n_slots; ++i) {
-        const Tile &T = tiles[size_t(i)];
-        o_ch[size_t(i) + 1] = o_ch[size_t(i)] + int64_t(T.chunks.size());
+        const BinTile &T = tiles[size_t(i)];
         o_px[size_t(i) + 1] = o_px[size_t(i)] + int64_t(T.px.size());
         o_pr[size_t(i) + 1] = o_pr[size_t(i)] + int64_t(T.pairs.size());
     }
@@ -1260,21 +1330,15 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
         fail(DG_UNSUPPORTED, "table too large for bin tiles");
     // default-initialised (not zeroed): every element is written below
     const size_t n_chunks = size_t(o_ch[size_t(n_slots)]), n_pairs = size_t(o_pr[size_t(n_slots)]);
-    const size_t n_pieces = order.size();
-    std::vector<int4> items(n_pieces), org(static_cast<size_t>(nb));
+    const std::vector<int4> &items = layout.items;
+    std::vector<int4> org(static_cast<size_t>(nb));
     // per row {origin entry, first valid entry, row end, 0} (row_origin)
     for (int64_t r = 0; r < nb; ++r)
         org[size_t(r)] = make_int4(oe[size_t(r)], fv[size_t(r)], int(rp[size_t(r) + 1]), 0);
     std::unique_ptr<int32_t[]> meta(new int32_t[std::max<size_t>(n_chunks * kBtMetaWords, 1)]);
     std::unique_ptr<int4[]> pairs(new int4[std::max<size_t>(n_pairs, 1)]);
-    for (size_t i = 0; i < n_pieces; ++i) {
-        const Piece &p = *order[i];
-        const int64_t r0 = p.tile * kBtRows;
-        items[i] = make_int4(int(r0), int(std::min<int64_t>(nb, r0 + kBtRows) - r0),
-                             int(o_ch[size_t(p.tile)]) + p.c0, p.n);
-    }
     auto flatten = [&](int64_t i) {
-        Tile &T = tiles[size_t(i)];
+        BinTile &T = tiles[size_t(i)];
         const int64_t c0 = o_ch[size_t(i)], pr0 = o_pr[size_t(i)];
         for (size_t c = 0; c < T.chunks.size(); ++c) {
             const int4 ch = T.chunks[c];
@@ -1289,47 +1353,28 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
             std::fill(rec + kBtMetaHead + ch.y, rec + kBtMetaWords, 0);
         }
         std::copy(T.pairs.begin(), T.pairs.end(), pairs.get() + pr0);
-        T = Tile();
+        T = BinTile();
     };
-    parallel(flatten, n_slots);
+    parallel(n_slots, flatten);
     out.n_items = int32_t(items.size());
     out.item.alloc(items.size());
     out.counter.alloc(2);
     DG_CUDA(cudaMemsetAsync(out.counter.ptr, 0, out.counter.bytes(), s));
     if (out.split) {
-        // Spans per item and row, and the pieces of every row in tile order
-        // (partial sums are kept per item and row).
-        std::vector<int4> spans[2];
-        std::vector<std::vector<int32_t>> slot(static_cast<size_t>(n_items));
-        for (int64_t ti = 0; ti < n_items; ++ti) slot[size_t(ti)].resize(cut[size_t(ti)].size());
-        for (size_t i = 0; i < n_pieces; ++i) {
-            const Piece &p = *order[i];
-            slot[size_t(p.tile)][size_t(order[i] - cut[size_t(p.tile)].data())] = int32_t(i);
-            for (int s2 = 0; s2 < 2; ++s2) {
-                if (p.spans[s2].empty())  // an uncut tile
-                    spans[s2].insert(spans[s2].end(), size_t(kBtRows), make_int4(0, 0, INT_MAX, 0));
-                else
-                    spans[s2].insert(spans[s2].end(), p.spans[s2].begin(), p.spans[s2].end());
-            }
-        }
-        std::vector<int32_t> row_part(size_t(nb) + 1, 0), ids;
-        for (int64_t r = 0; r < nb; ++r) {
-            for (int32_t i : slot[size_t(r / kBtRows)]) ids.push_back(i * kBtRows + int32_t(r % kBtRows));
-            row_part[size_t(r) + 1] = int32_t(ids.size());
-        }
+        const std::vector<int4>(&spans)[2] = layout.spans;
+        const std::vector<int32_t> &row_part = layout.row_part, &ids = layout.part_ids;
         for (int s2 = 0; s2 < 2; ++s2) {
             out.span[s2].alloc(spans[s2].size());
             DG_CUDA(cudaMemcpyAsync(out.span[s2].ptr, spans[s2].data(), spans[s2].size() * sizeof(int4),
                                     cudaMemcpyHostToDevice, s));
         }
-        out.tile_done.alloc(size_t(n_items) * size_t(256 / CFG::kFrames));
+        out.tile_done.alloc(tiles.size() * size_t(256 / CFG::kFrames));
         DG_CUDA(cudaMemsetAsync(out.tile_done.ptr, 0, out.tile_done.bytes(), s));
         out.row_part.alloc(row_part.size());
         out.part_ids.alloc(ids.size());
         DG_CUDA(cudaMemcpyAsync(out.row_part.ptr, row_part.data(), row_part.size() * 4,
                                 cudaMemcpyHostToDevice, s));
         DG_CUDA(cudaMemcpyAsync(out.part_ids.ptr, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, s));
-        DG_CUDA(cudaStreamSynchronize(s));  // the lists are local
     }
     out.meta.alloc(std::max<size_t>(n_chunks * kBtMetaWords, 1));
     out.org.alloc(org.size());
@@ -1361,6 +1406,20 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
     // Only mapping 8's tiles carry per-frame masks; the others drop the
     // descriptor once their pairs are filled.
     if (!std::is_same<CFG, Bt8>::value) desc.release();
+}
+
+void bin_items(int variant, int64_t n_rows, const int64_t *row_ptr, const int32_t *col,
+               BinItems &out) {
+    BinLayout layout;
+    if (variant == 7) lay_out_bin_tiles<Bt7>(row_ptr, col, n_rows, layout);
+    else if (variant == 8) lay_out_bin_tiles<Bt8>(row_ptr, col, n_rows, layout);
+    else fail(DG_INVALID_INPUT, "bin tiles are lane mappings 7 and 8");
+    out.rows = variant == 7 ? Bt7::kRows : Bt8::kRows;
+    out.first_chunk = std::move(layout.first_chunk);
+    out.items = std::move(layout.items);
+    for (int s2 = 0; s2 < 2; ++s2) out.spans[s2] = std::move(layout.spans[s2]);
+    out.row_part = std::move(layout.row_part);
+    out.part_ids = std::move(layout.part_ids);
 }
 
 bool bin_tile_wait_failed(const GatherTable &t) {

@@ -447,6 +447,17 @@ void flip_gather_rows(GatherTable &t, int32_t dim1, int32_t dim2, cudaStream_t s
 // table on first use (the autotuner, or selecting the mapping); idempotent.
 void ensure_bin_tiles(GatherTable &t, const DeviceCsr &table, int variant, cudaStream_t s);
 bool gather_variant_needs_tiles(int variant);
+// The work items of bin tiles 7 or 8 for a table in host memory, as
+// ensure_bin_tiles makes them (dg_test_bin_items).
+struct BinItems {
+    int rows = 0;                             // rows per tile
+    std::vector<int64_t> first_chunk;         // per tile, then the number of chunks
+    std::vector<int4> items;                  // {first row, rows, first chunk, chunks}
+    std::vector<int4> spans[2];               // as BinTiles::span; empty where no tile is cut
+    std::vector<int32_t> row_part, part_ids;
+};
+void bin_items(int variant, int64_t n_rows, const int64_t *row_ptr, const int32_t *col,
+               BinItems &out);
 // Frame-lane units of mappings 5 and 6, built on first use; idempotent.
 void ensure_fl_units(GatherTable &t, const DeviceCsr &table, cudaStream_t s);
 // Throws DG_TIMEOUT (once) when a bin-tile launch of this table gave up a
