@@ -498,7 +498,7 @@ dg_status dg_plan_test_wait_timeout(dg_plan *plan, const void *d_frames, int32_t
 }
 
 dg_status dg_test_bin_items(int32_t variant, int64_t n_rows, const int64_t *row_ptr,
-                            const int32_t *col, int64_t counts[4], int32_t *items,
+                            const int32_t *col, int64_t counts[5], int32_t *items,
                             int64_t *first_chunk, int32_t *spans, int32_t *row_part,
                             int32_t *part_ids) {
     return guarded([&] {
@@ -510,6 +510,7 @@ dg_status dg_test_bin_items(int32_t variant, int64_t n_rows, const int64_t *row_
         counts[1] = b.rows;
         counts[2] = int64_t(b.first_chunk.size()) - 1;
         counts[3] = int64_t(b.part_ids.size());
+        counts[4] = b.partial_rows;
         auto put = [](const auto &v, auto *out) {
             if (out && !v.empty()) std::memcpy(out, v.data(), v.size() * sizeof v[0]);
         };

@@ -275,11 +275,11 @@ struct BinArgs {
     int32_t n_frames, n_rows, n_items, groups;
     int32_t *counter;    // {next claim, CTAs done}, both 0 between launches
     double *out_i, *out_s, *out_d, *out_c;
-    // With spans: partial sums [item row][accumulator][frame], every row's item
-    // rows (the table's in row_part), and the pieces done per (tile, group), 0
-    // between launches.
+    // With spans: partial sums [slot row][accumulator][frame], the slots of the
+    // items, every row's slot rows (the table's in row_part), and the pieces done
+    // per (tile, group), 0 between launches.
     double *partial;
-    const int32_t *row_part, *part_ids;
+    const int32_t *slot, *row_part, *part_ids;
     int32_t *tile_done;
     const double *raw_cnt;
     const uint64_t *mask_words;  // per group and pixel: bit f masks frame f of the group
@@ -786,11 +786,12 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
         const int pieces = a.spans ? a.row_part[it.x + 1] - a.row_part[it.x] : 1;
         if (pieces > 1) {
             if (mine) {
+                const int64_t slot = a.slot[item];
 #pragma unroll
                 for (int h = 0; h < F2; ++h) {
                     const int fl = lane + 32 * h;
                     if (fl >= nv) continue;
-                    double *o = a.partial + (int64_t(item) * NW + r) * NA * a.n_frames + f0 + fl;
+                    double *o = a.partial + (slot * NW + r) * NA * a.n_frames + f0 + fl;
 #pragma unroll
                     for (int k = 0; k < NA; ++k) __stcg(o + int64_t(k) * a.n_frames, v[h][k]);
                 }
@@ -1011,6 +1012,10 @@ struct BinLayout {
     bool split = false;                       // with the lists below
     std::vector<int4> spans[2];               // per item and row
     std::vector<int32_t> row_part, part_ids;  // every row's pieces (item * kRows + row), in order
+    // Per item its slot among the pieces of cut tiles (-1: an uncut tile, which
+    // leaves no partial sums), and the number of slots.
+    std::vector<int32_t> slot;
+    int32_t n_slots = 0;
 };
 
 // fn(0) .. fn(count - 1) over host threads.
@@ -1273,12 +1278,13 @@ void lay_out_bin_tiles(const int64_t *rp, const int32_t *col, int64_t nb, BinLay
     }
     if (!out.split) return;
     // Spans per item and row, and the pieces of every row in tile order
-    // (partial sums are kept per item and row).
-    std::vector<std::vector<int32_t>> slot(static_cast<size_t>(n_items));
-    for (int64_t ti = 0; ti < n_items; ++ti) slot[size_t(ti)].resize(cut[size_t(ti)].size());
+    // (partial sums are kept per piece of a cut tile and row).
+    std::vector<std::vector<int32_t>> pieces(static_cast<size_t>(n_items));
+    for (int64_t ti = 0; ti < n_items; ++ti) pieces[size_t(ti)].resize(cut[size_t(ti)].size());
     for (size_t i = 0; i < order.size(); ++i) {
         const BinPiece &p = *order[i];
-        slot[size_t(p.tile)][size_t(order[i] - cut[size_t(p.tile)].data())] = int32_t(i);
+        out.slot.push_back(cut[size_t(p.tile)].size() > 1 ? out.n_slots++ : -1);
+        pieces[size_t(p.tile)][size_t(order[i] - cut[size_t(p.tile)].data())] = int32_t(i);
         for (int s2 = 0; s2 < 2; ++s2) {
             if (p.spans[s2].empty())  // an uncut tile
                 out.spans[s2].insert(out.spans[s2].end(), size_t(kBtRows), make_int4(0, 0, INT_MAX, 0));
@@ -1288,7 +1294,7 @@ void lay_out_bin_tiles(const int64_t *rp, const int32_t *col, int64_t nb, BinLay
     }
     out.row_part.assign(size_t(nb) + 1, 0);
     for (int64_t r = 0; r < nb; ++r) {
-        for (int32_t i : slot[size_t(r / kBtRows)])
+        for (int32_t i : pieces[size_t(r / kBtRows)])
             out.part_ids.push_back(i * kBtRows + int32_t(r % kBtRows));
         out.row_part[size_t(r) + 1] = int32_t(out.part_ids.size());
     }
@@ -1362,7 +1368,15 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
     DG_CUDA(cudaMemsetAsync(out.counter.ptr, 0, out.counter.bytes(), s));
     if (out.split) {
         const std::vector<int4>(&spans)[2] = layout.spans;
-        const std::vector<int32_t> &row_part = layout.row_part, &ids = layout.part_ids;
+        const std::vector<int32_t> &row_part = layout.row_part;
+        // the pieces' partial sums: slot * rows + row of the tile
+        std::vector<int32_t> ids(layout.part_ids);
+        for (int32_t &id : ids)
+            id = std::max(0, layout.slot[size_t(id / kBtRows)]) * kBtRows + id % kBtRows;
+        out.partial_rows = int64_t(layout.n_slots) * kBtRows;
+        out.slot.alloc(layout.slot.size());
+        DG_CUDA(cudaMemcpyAsync(out.slot.ptr, layout.slot.data(), layout.slot.size() * 4,
+                                cudaMemcpyHostToDevice, s));
         for (int s2 = 0; s2 < 2; ++s2) {
             out.span[s2].alloc(spans[s2].size());
             DG_CUDA(cudaMemcpyAsync(out.span[s2].ptr, spans[s2].data(), spans[s2].size() * sizeof(int4),
@@ -1375,6 +1389,7 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
         DG_CUDA(cudaMemcpyAsync(out.row_part.ptr, row_part.data(), row_part.size() * 4,
                                 cudaMemcpyHostToDevice, s));
         DG_CUDA(cudaMemcpyAsync(out.part_ids.ptr, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, s));
+        DG_CUDA(cudaStreamSynchronize(s));  // ids is local
     }
     out.meta.alloc(std::max<size_t>(n_chunks * kBtMetaWords, 1));
     out.org.alloc(org.size());
@@ -1420,6 +1435,7 @@ void bin_items(int variant, int64_t n_rows, const int64_t *row_ptr, const int32_
     for (int s2 = 0; s2 < 2; ++s2) out.spans[s2] = std::move(layout.spans[s2]);
     out.row_part = std::move(layout.row_part);
     out.part_ids = std::move(layout.part_ids);
+    out.partial_rows = int64_t(layout.n_slots) * out.rows;
 }
 
 bool bin_tile_wait_failed(const GatherTable &t) {
@@ -1505,6 +1521,7 @@ void launch(const GatherTable &t, const BinTiles &bt, const BinCall &c, cudaStre
     a.out_d = c.out_d;
     a.out_c = c.out_c;
     a.partial = c.partial;
+    a.slot = bt.slot.ptr;
     a.row_part = bt.row_part.ptr;
     a.part_ids = bt.part_ids.ptr;
     a.tile_done = bt.tile_done.ptr;
@@ -1544,8 +1561,7 @@ void launch_typed(const GatherTable &t, int variant, const BinCall &c, cudaStrea
 }  // namespace
 
 int64_t bin_tile_partials(const GatherTable &t, int variant) {
-    const BinTiles &bt = t.bt[variant - 7];
-    return bt.split ? int64_t(bt.n_items) * (variant == 7 ? Bt7::kRows : Bt8::kRows) : 0;
+    return t.bt[variant - 7].partial_rows;
 }
 
 void launch_bin_tiles(GatherTable &t, int variant, const BinCall &c, cudaStream_t s) {

@@ -253,12 +253,13 @@ struct BinTiles {
     int32_t n_items = 0;
     DeviceArray<int4> item;        // {first row, rows, first chunk, chunks}, largest first
     // Large tiles cut into pieces (items): per item and row the {chunk, pair}
-    // it starts and ends at, for both fold cadences, and every row's partial
-    // sums (item * rows + row of the tile) in order.
+    // it starts and ends at, for both fold cadences, the items' slots (-1: a whole
+    // tile), and every row's partial sums (slot * rows + row of the tile) in order.
     bool split = false;
+    int64_t partial_rows = 0;      // slots * rows
     DeviceArray<int32_t> counter;  // a launch's next claim and finished CTAs
     DeviceArray<int4> span[2];
-    DeviceArray<int32_t> row_part, part_ids;
+    DeviceArray<int32_t> slot, row_part, part_ids;
     DeviceArray<int32_t> tile_done;     // pieces done per (tile, frame group) of a launch
     mutable bool unfinished = false;    // a launch gave up: counters to reset
     DeviceArray<int32_t> meta;     // per chunk: {pixels, pairs, first pair}, row offsets, pixels
@@ -273,7 +274,7 @@ struct BinTiles {
     // Set by k_gather_bins when a wait of its chunk pipeline gave up.
     PinnedFlag wait_err;
     int64_t bytes() const {
-        return int64_t(span[0].bytes() + span[1].bytes() + row_part.bytes() + part_ids.bytes() + tile_done.bytes() + counter.bytes() +
+        return int64_t(span[0].bytes() + span[1].bytes() + slot.bytes() + row_part.bytes() + part_ids.bytes() + tile_done.bytes() + counter.bytes() +
                        item.bytes() + meta.bytes() + org.bytes() + pair_a.bytes() +
                        pair_as.bytes() + pair_b.bytes() + pair_c.bytes() + desc.bytes() + pair_ra.bytes() +
                        pair_rb.bytes());
@@ -455,6 +456,7 @@ struct BinItems {
     std::vector<int4> items;                  // {first row, rows, first chunk, chunks}
     std::vector<int4> spans[2];               // as BinTiles::span; empty where no tile is cut
     std::vector<int32_t> row_part, part_ids;
+    int64_t partial_rows = 0;                 // rows of partial sums a launch keeps
 };
 void bin_items(int variant, int64_t n_rows, const int64_t *row_ptr, const int32_t *col,
                BinItems &out);

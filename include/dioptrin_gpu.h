@@ -203,14 +203,14 @@ DG_EXPORT dg_status dg_plan_test_wait_timeout(dg_plan *plan, const void *d_frame
 
 /* Test hook, host memory only (no GPU): the work items that bin-tile mapping
  * `variant` (7 or 8) makes of a table of n_rows rows. counts receives {items,
- * rows per tile, tiles, part ids or 0 where no tile is cut}; arrays that are NULL are skipped, so
- * a first call gives the sizes. items: {first row, rows, first chunk, chunks}
+ * rows per tile, tiles, part ids or 0 where no tile is cut, rows of partial sums};
+ * arrays that are NULL are skipped, so a first call gives the sizes. items: {first row, rows, first chunk, chunks}
  * each; first_chunk: per tile, then the number of chunks; spans: for the two
  * fold cadences, per item and row of the tile the {chunk, pair} to start and to
  * end at, chunks relative to the item's first; row_part (n_rows + 1) and part_ids:
  * every row's pieces (item * rows per tile + row of the tile) in order. */
 DG_EXPORT dg_status dg_test_bin_items(int32_t variant, int64_t n_rows, const int64_t *row_ptr,
-                                      const int32_t *col, int64_t counts[4], int32_t *items,
+                                      const int32_t *col, int64_t counts[5], int32_t *items,
                                       int64_t *first_chunk, int32_t *spans, int32_t *row_part,
                                       int32_t *part_ids);
 

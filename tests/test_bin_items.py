@@ -17,7 +17,7 @@ def bin_items(variant, row_ptr, col):
     rp = np.ascontiguousarray(row_ptr, np.int64)
     col = np.ascontiguousarray(col, np.int32)
     n = len(rp) - 1
-    counts = np.zeros(4, np.int64)
+    counts = np.zeros(5, np.int64)
 
     def call(*arrays):
         N.check(N.lib().dg_test_bin_items(
@@ -25,7 +25,7 @@ def bin_items(variant, row_ptr, col):
             *[a.ctypes.data if a is not None else None for a in arrays]))
 
     call(*[None] * 5)
-    items, rows, tiles, parts = (int(v) for v in counts)
+    items, rows, tiles, parts, _ = (int(v) for v in counts)
     out = dict(rows=rows, items=np.zeros((items, 4), np.int32),
                first_chunk=np.zeros(tiles + 1, np.int64),
                spans=np.zeros((2, items, rows, 4), np.int32),
