@@ -1364,8 +1364,10 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
     parallel(n_slots, flatten);
     out.n_items = int32_t(items.size());
     out.item.alloc(items.size());
-    out.counter.alloc(2);
-    DG_CUDA(cudaMemsetAsync(out.counter.ptr, 0, out.counter.bytes(), s));
+    for (auto &n : out.counts) {
+        n.claim.alloc(2);
+        DG_CUDA(cudaMemsetAsync(n.claim.ptr, 0, n.claim.bytes(), s));
+    }
     if (out.split) {
         const std::vector<int4>(&spans)[2] = layout.spans;
         const std::vector<int32_t> &row_part = layout.row_part;
@@ -1382,8 +1384,10 @@ void build_bin_tiles(GatherTable &gt, BinTiles &out, const DeviceCsr &table, cud
             DG_CUDA(cudaMemcpyAsync(out.span[s2].ptr, spans[s2].data(), spans[s2].size() * sizeof(int4),
                                     cudaMemcpyHostToDevice, s));
         }
-        out.tile_done.alloc(tiles.size() * size_t(256 / CFG::kFrames));
-        DG_CUDA(cudaMemsetAsync(out.tile_done.ptr, 0, out.tile_done.bytes(), s));
+        for (auto &n : out.counts) {
+            n.tile_done.alloc(tiles.size() * size_t(256 / CFG::kFrames));
+            DG_CUDA(cudaMemsetAsync(n.tile_done.ptr, 0, n.tile_done.bytes(), s));
+        }
         out.row_part.alloc(row_part.size());
         out.part_ids.alloc(ids.size());
         DG_CUDA(cudaMemcpyAsync(out.row_part.ptr, row_part.data(), row_part.size() * 4,
@@ -1443,7 +1447,7 @@ bool bin_tile_wait_failed(const GatherTable &t) {
     for (const BinTiles &bt : t.bt)
         if (bt.wait_err.host && *static_cast<volatile int *>(bt.wait_err.host)) {
             *bt.wait_err.host = 0;
-            bt.unfinished = true;
+            bt.counts[0].unfinished = bt.counts[1].unfinished = true;
             failed = true;
         }
     return failed;
@@ -1515,7 +1519,13 @@ void launch(const GatherTable &t, const BinTiles &bt, const BinCall &c, cudaStre
     a.n_rows = t.n_rows;
     a.n_items = bt.n_items;
     a.groups = (c.n_frames + CFG::kFrames - 1) / CFG::kFrames;
-    a.counter = bt.counter.ptr;
+    // Counts: a replay of a captured launch is ordered by its caller alone, and is
+    // preceded by its own reset, since no call of the library comes before it.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    DG_CUDA(cudaStreamIsCapturing(s, &capture));
+    const bool captured = capture != cudaStreamCaptureStatusNone;
+    const BinTiles::Counts &counts = bt.counts[c.fixed || captured ? 1 : 0];
+    a.counter = counts.claim.ptr;
     a.out_i = c.out_i;
     a.out_s = c.out_s;
     a.out_d = c.out_d;
@@ -1524,7 +1534,7 @@ void launch(const GatherTable &t, const BinTiles &bt, const BinCall &c, cudaStre
     a.slot = bt.slot.ptr;
     a.row_part = bt.row_part.ptr;
     a.part_ids = bt.part_ids.ptr;
-    a.tile_done = bt.tile_done.ptr;
+    a.tile_done = counts.tile_done.ptr;
     a.raw_cnt = t.cnt.ptr;
     a.raw = c.raw;
     a.mask_words = t.mask_words.ptr;
@@ -1533,10 +1543,11 @@ void launch(const GatherTable &t, const BinTiles &bt, const BinCall &c, cudaStre
     if (int64_t(a.n_items) * a.groups > INT32_MAX)
         fail(DG_UNSUPPORTED, "too many bin tiles for one launch");
     check_bin_tile_waits(t);
-    if (bt.unfinished) {  // a launch that gave up left tiles partly done
-        DG_CUDA(cudaMemsetAsync(bt.counter.ptr, 0, bt.counter.bytes(), s));
-        if (bt.split) DG_CUDA(cudaMemsetAsync(bt.tile_done.ptr, 0, bt.tile_done.bytes(), s));
-        bt.unfinished = false;
+    if (counts.unfinished || captured) {  // a launch that gave up left tiles partly done
+        DG_CUDA(cudaMemsetAsync(counts.claim.ptr, 0, counts.claim.bytes(), s));
+        if (bt.split)
+            DG_CUDA(cudaMemsetAsync(counts.tile_done.ptr, 0, counts.tile_done.bytes(), s));
+        if (!captured) counts.unfinished = false;
     }
     const int grid = std::min(a.n_items * a.groups, sm_count());
     kern<<<unsigned(grid), CFG::template threads<MODE, P>(), smem, s>>>(a);

@@ -1688,6 +1688,7 @@ bool launch_gather(GatherTable &t, int variant, const P *fp, int64_t n_pixels, i
                 c.out_s = os;
                 c.out_d = od;
                 c.partial = partial;
+                c.fixed = partial != t.partial.ptr;
                 launch_bin_tiles(t, variant, c, s);
                 return true;
             }
@@ -2198,9 +2199,10 @@ void run_gather(GatherTable &t, const void *d_frames, int dtype, int64_t n_pixel
             reserve_partials(t, std::min<int64_t>(chunk, n_frames), flags, dtype);
         partial = t.partial.ptr;
     }
-    // The plan's partial sums and the bin tiles' item counter are shared by its
-    // calls; row warps share nothing.
-    const bool shared = gather_variant_needs_tiles(t.variant) || (!scratch && partial_rows(t) > 0);
+    // The plan's partial sums and the bin tiles' counts are shared by its calls;
+    // row warps share nothing. Calls with a fixed scratch have counts of their own
+    // and are ordered by their caller: an event of another stream would end a capture.
+    const bool shared = !scratch && (gather_variant_needs_tiles(t.variant) || partial_rows(t) > 0);
     if (shared) t.scratch.wait(s);
     const size_t esize = dtype == DG_U16 ? 2 : dtype == DG_F64 ? 8 : 4;
     for (int64_t f0 = 0; f0 < n_frames; f0 += chunk) {

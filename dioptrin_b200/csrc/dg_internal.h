@@ -257,11 +257,16 @@ struct BinTiles {
     // tile), and every row's partial sums (slot * rows + row of the tile) in order.
     bool split = false;
     int64_t partial_rows = 0;      // slots * rows
-    DeviceArray<int32_t> counter;  // a launch's next claim and finished CTAs
+    // What a launch counts in, 0 between launches: its next claim and finished CTAs,
+    // and the pieces done per (tile, frame group). [0] belongs to the calls that the
+    // plan orders (ScratchOrder); [1] to those that their caller orders, which are the
+    // calls with a fixed scratch and the replays of a captured graph.
+    struct Counts {
+        DeviceArray<int32_t> claim, tile_done;
+        mutable bool unfinished = false;  // a launch gave up: to be reset
+    } counts[2];
     DeviceArray<int4> span[2];
     DeviceArray<int32_t> slot, row_part, part_ids;
-    DeviceArray<int32_t> tile_done;     // pieces done per (tile, frame group) of a launch
-    mutable bool unfinished = false;    // a launch gave up: counters to reset
     DeviceArray<int32_t> meta;     // per chunk: {pixels, pairs, first pair}, row offsets, pixels
     DeviceArray<int4> org;         // per row {origin entry, first valid entry, row end, 0}
     DeviceArray<float4> pair_a, pair_as, pair_b;
@@ -274,7 +279,8 @@ struct BinTiles {
     // Set by k_gather_bins when a wait of its chunk pipeline gave up.
     PinnedFlag wait_err;
     int64_t bytes() const {
-        return int64_t(span[0].bytes() + span[1].bytes() + slot.bytes() + row_part.bytes() + part_ids.bytes() + tile_done.bytes() + counter.bytes() +
+        return int64_t(span[0].bytes() + span[1].bytes() + slot.bytes() + row_part.bytes() + part_ids.bytes() + counts[0].claim.bytes() +
+                       counts[0].tile_done.bytes() + counts[1].claim.bytes() + counts[1].tile_done.bytes() +
                        item.bytes() + meta.bytes() + org.bytes() + pair_a.bytes() +
                        pair_as.bytes() + pair_b.bytes() + pair_c.bytes() + desc.bytes() + pair_ra.bytes() +
                        pair_rb.bytes());
@@ -357,7 +363,8 @@ void make_gather_table(const DeviceCsr &table, const double *d_norm, int32_t dim
 // Enqueues the batched gather for n_frames device-resident frames. With
 // `scratch` (scratch_doubles long) the partial sums go there instead of the
 // plan's own array, which is then neither allocated nor ordered across
-// streams; frames per launch shrink to what the scratch holds.
+// streams (no event is waited for or recorded: the caller orders such calls, and
+// may capture them); frames per launch shrink to what the scratch holds.
 void run_gather(GatherTable &t, const void *d_frames, int dtype, int64_t n_pixels,
                 int64_t n_frames, uint32_t flags, int precision, double *d_i, double *d_sigma,
                 double *d_std, cudaStream_t stream, double *scratch = nullptr,
@@ -379,6 +386,7 @@ struct BinCall {
     const uint8_t *masks;         // per-frame masks (mapping 8)
     int64_t mask_stride;
     double *partial;
+    bool fixed;                   // partial is a fixed scratch, not the plan's
 };
 void launch_bin_tiles(GatherTable &t, int variant, const BinCall &c, cudaStream_t s);
 // Partial sums per frame and accumulator of bin tiles 7 or 8 (0: none).

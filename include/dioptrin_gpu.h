@@ -171,9 +171,12 @@ DG_EXPORT dg_status dg_integrate_device(dg_plan *plan, const void *d_frames, int
  * sums for a single frame exceed the array is rejected with
  * DG_UNSUPPORTED (row warps keep none, bin tiles some 0.2 MiB per frame for the
  * tiles they cut). The first call on a device looks up the array's device
- * address (cudaGetSymbolAddress); make it before any stream capture. All
- * calls on a device share the array, so calls that overlap on the GPU race:
- * serialise them. Results equal dg_integrate_device's. */
+ * address (cudaGetSymbolAddress); make it before any stream capture. The call
+ * waits for no event and records none, so it can be captured on any stream, and a
+ * replay runs beside dg_integrate_device calls on the same plan. All
+ * allocation-free calls on a device (replays among them) share the array, so
+ * those that overlap on the GPU race: serialise them. Results equal
+ * dg_integrate_device's. */
 DG_EXPORT dg_status dg_integrate_device_noalloc(dg_plan *plan, const void *d_frames,
                                                 int32_t dtype, int64_t n_frames, uint32_t flags,
                                                 double *d_intensity, double *d_sigma,
