@@ -14,8 +14,11 @@
 // stream alone and synchronise it before any other stream sees what they leave.
 // Outside a scope an allocation is complete when the call returns, and a free
 // waits for the device first, as cudaFree does: arrays of a living plan may be
-// in use on any of the callers' streams.
+// in use on any of the callers' streams. The wait is a cudaFree (device_wait):
+// cudaDeviceSynchronize would end every stream capture in the process, of other
+// threads and of relaxed mode too, and then not have waited.
 #include <mutex>
+#include <vector>
 
 #include "dg_internal.h"
 
@@ -30,6 +33,8 @@ struct Pool {
     cudaError_t error = cudaSuccess;
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;  // order of allocations outside a scope
+    std::mutex mu;
+    std::vector<void *> pending;    // to be freed after the next wait for the device
 };
 
 // One per device for the life of the process; the device must be current.
@@ -48,6 +53,8 @@ Pool *pool_of(int device) {
             p.error = cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep);
         if (p.error == cudaSuccess)
             p.error = cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking);
+        void *small = nullptr;  // kept for device_wait
+        if (p.error == cudaSuccess) p.error = cudaMalloc(&small, 256);
     });
     return &p;
 }
@@ -60,7 +67,29 @@ cudaError_t take(Pool &p, void **out, size_t bytes) {
     return e == cudaSuccess ? cudaStreamSynchronize(p.stream) : e;
 }
 
+// Frees what earlier frees could not (a capture forbade the wait); after a wait.
+void free_pending(Pool &p) {
+    std::vector<void *> list;
+    {
+        std::lock_guard<std::mutex> lock(p.mu);
+        list.swap(p.pending);
+    }
+    for (void *ptr : list) (void)cudaFreeAsync(ptr, p.stream);
+}
+
 }  // namespace
+
+// 256 bytes of their own: cudaFree waits for all of the device's work, and both
+// calls take 2 to 4 us as long as another small block (pool_of's) keeps the
+// driver's chunk of them alive.
+bool device_wait() noexcept {
+    void *block = nullptr;
+    cudaError_t e = cudaMalloc(&block, 256);
+    if (e == cudaErrorMemoryAllocation) e = cudaDeviceSynchronize();
+    else if (e == cudaSuccess) e = cudaFree(block);
+    (void)cudaGetLastError();
+    return e == cudaSuccess;
+}
 
 AllocScope::AllocScope(cudaStream_t s) : stream(s), outer(t_scope) { t_scope = this; }
 AllocScope::~AllocScope() { t_scope = static_cast<const AllocScope *>(outer); }
@@ -83,7 +112,8 @@ void *device_alloc(size_t bytes, int *device) {
     cudaError_t e = take(*p, &ptr, bytes);
     if (e == cudaErrorMemoryAllocation) {  // give back what the pool holds and try again
         (void)cudaGetLastError();
-        (void)cudaDeviceSynchronize();
+        if (device_wait()) free_pending(*p);
+        (void)cudaStreamSynchronize(p->stream);
         (void)cudaMemPoolTrimTo(p->pool, 0);
         e = take(*p, &ptr, bytes);
     }
@@ -102,8 +132,20 @@ void device_free(void *ptr, int device) noexcept {
     if (previous != device) (void)cudaSetDevice(device);
     Pool *p = pool_of(device);
     if (p && p->error == cudaSuccess) {
-        if (!t_scope) (void)cudaDeviceSynchronize();
-        (void)cudaFreeAsync(ptr, t_scope ? t_scope->stream : p->stream);
+        bool freed = false;
+        if (t_scope) {
+            freed = cudaFreeAsync(ptr, t_scope->stream) == cudaSuccess;
+        } else if (device_wait()) {
+            free_pending(*p);
+            freed = cudaFreeAsync(ptr, p->stream) == cudaSuccess;
+        }
+        if (!freed) {  // a capture of this thread, or a global one, forbids it: later
+            try {
+                std::lock_guard<std::mutex> lock(p->mu);
+                p->pending.push_back(ptr);
+            } catch (...) {
+            }
+        }
     }
     if (previous != device) (void)cudaSetDevice(previous);
     (void)cudaGetLastError();

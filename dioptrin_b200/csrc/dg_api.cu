@@ -11,6 +11,7 @@
 #include <map>
 #include <memory>
 #include <new>
+#include <optional>
 
 #include "dg_internal.h"
 
@@ -313,9 +314,10 @@ dg_status dg_plan_destroy(dg_plan *plan) {
             cudaGetDevice(&prev);
             cudaSetDevice(plan->device);
             // Callers' streams may still run on the tables: wait for them once,
-            // then every array is freed without waiting.
-            (void)cudaDeviceSynchronize();
-            dg::AllocScope alloc(dg::idle_stream());
+            // then every array is freed without waiting (or, where a capture
+            // forbids the wait, kept by the pool until one is possible).
+            std::optional<dg::AllocScope> alloc;
+            if (dg::device_wait()) alloc.emplace(dg::idle_stream());
             plan->full = dg::DeviceCsr();
             plan->table = dg::DeviceCsr();
             plan->norm.release();

@@ -31,6 +31,9 @@ void check_cuda(cudaError_t err, const char *what);
 // the device first.
 void *device_alloc(size_t bytes, int *device);
 void device_free(void *ptr, int device) noexcept;
+// Waits for all work of the current device, as cudaFree does; false where a stream
+// capture forbids it.
+bool device_wait() noexcept;
 struct AllocScope {
     cudaStream_t stream;
     const void *outer;
