@@ -1,4 +1,4 @@
-// Device memory of plans, from one stream-ordered pool per device.
+// Device memory of plans, from one stream-ordered pool per device and context.
 //
 // A plan's creation and its destruction make about fifty-five allocations and
 // as many frees. cudaMalloc took 0.35 ms and cudaFree 0.30 ms each on a B200
@@ -17,6 +17,9 @@
 // in use on any of the callers' streams. The wait is a cudaFree (device_wait):
 // cudaDeviceSynchronize would end every stream capture in the process, of other
 // threads and of relaxed mode too, and then not have waited.
+#include <cuda.h>
+
+#include <map>
 #include <mutex>
 #include <vector>
 
@@ -26,37 +29,77 @@ namespace dg {
 namespace {
 
 constexpr uint64_t kPoolKeep = uint64_t(1) << 30;
-constexpr int kMaxDevices = 64;
 
 struct Pool {
-    std::once_flag once;
-    cudaError_t error = cudaSuccess;
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;  // order of allocations outside a scope
     std::mutex mu;
     std::vector<void *> pending;    // to be freed after the next wait for the device
 };
 
-// One per device for the life of the process; the device must be current.
-Pool *pool_of(int device) {
-    static Pool *const pools = new Pool[kMaxDevices];  // not destroyed: arrays may outlive statics
-    if (device < 0 || device >= kMaxDevices) return nullptr;
-    Pool &p = pools[device];
-    std::call_once(p.once, [&] {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        p.error = cudaMemPoolCreate(&p.pool, &props);
-        uint64_t keep = kPoolKeep;
-        if (p.error == cudaSuccess)
-            p.error = cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        if (p.error == cudaSuccess)
-            p.error = cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking);
-        void *small = nullptr;  // kept for device_wait
-        if (p.error == cudaSuccess) p.error = cudaMalloc(&small, 256);
-    });
+// Number of the current CUDA context, which no later one of the process has: a
+// pool and its stream end with their context (cudaDeviceReset), and a new context
+// gets new ones. 0 where the driver does not tell.
+uint64_t context_number() {
+    using Current = CUresult (*)(CUcontext *);
+    using Id = CUresult (*)(CUcontext, unsigned long long *);
+    static const std::pair<Current, Id> entry = [] {
+        void *current = nullptr, *id = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &current, cudaEnableDefault, &found) != cudaSuccess ||
+            cudaGetDriverEntryPoint("cuCtxGetId", &id, cudaEnableDefault, &found) != cudaSuccess)
+            current = id = nullptr;
+        (void)cudaGetLastError();
+        return std::make_pair(reinterpret_cast<Current>(current), reinterpret_cast<Id>(id));
+    }();
+    CUcontext context = nullptr;
+    unsigned long long number = 0;
+    if (!entry.first || !entry.second || entry.first(&context) != CUDA_SUCCESS) return 0;
+    if (!context) {  // the runtime makes the device's context with its first use
+        (void)cudaFree(nullptr);
+        if (entry.first(&context) != CUDA_SUCCESS || !context) return 0;
+    }
+    return entry.second(context, &number) == CUDA_SUCCESS ? number : 0;
+}
+
+// The pool of the current device and context, made on first use (and tried again
+// after a failure); nullptr and the error where it cannot be.
+Pool *pool_of(int device, uint64_t context, cudaError_t *error) {
+    // not destroyed: arrays may outlive statics
+    static auto *const mu = new std::mutex;
+    static auto *const pools = new std::map<std::pair<int, uint64_t>, Pool>;
+    std::lock_guard<std::mutex> lock(*mu);
+    Pool &p = (*pools)[{device, context}];
+    *error = cudaSuccess;
+    if (p.stream) return &p;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;
+    void *small = nullptr;  // kept for device_wait
+    uint64_t keep = kPoolKeep;
+    *error = cudaMemPoolCreate(&pool, &props);
+    if (*error == cudaSuccess)
+        *error = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (*error == cudaSuccess) *error = cudaMalloc(&small, 256);
+    if (*error == cudaSuccess) *error = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+    if (*error != cudaSuccess) {
+        (void)cudaFree(small);
+        if (pool) (void)cudaMemPoolDestroy(pool);
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    p.pool = pool;
+    p.stream = stream;
     return &p;
+}
+Pool &pool_of(int device, uint64_t context) {
+    cudaError_t e;
+    Pool *p = pool_of(device, context, &e);
+    DG_CUDA(e);
+    return *p;
 }
 
 thread_local const AllocScope *t_scope = nullptr;
@@ -97,25 +140,21 @@ AllocScope::~AllocScope() { t_scope = static_cast<const AllocScope *>(outer); }
 cudaStream_t idle_stream() {
     int device = 0;
     DG_CUDA(cudaGetDevice(&device));
-    Pool *p = pool_of(device);
-    if (!p) fail(DG_DEVICE, "device ordinal out of range");
-    DG_CUDA(p->error);
-    return p->stream;
+    return pool_of(device, context_number()).stream;
 }
 
-void *device_alloc(size_t bytes, int *device) {
+void *device_alloc(size_t bytes, int *device, uint64_t *context) {
     DG_CUDA(cudaGetDevice(device));
-    Pool *p = pool_of(*device);
-    if (!p) fail(DG_DEVICE, "device ordinal out of range");
-    DG_CUDA(p->error);
+    *context = context_number();
+    Pool &p = pool_of(*device, *context);
     void *ptr = nullptr;
-    cudaError_t e = take(*p, &ptr, bytes);
+    cudaError_t e = take(p, &ptr, bytes);
     if (e == cudaErrorMemoryAllocation) {  // give back what the pool holds and try again
         (void)cudaGetLastError();
-        if (device_wait()) free_pending(*p);
-        (void)cudaStreamSynchronize(p->stream);
-        (void)cudaMemPoolTrimTo(p->pool, 0);
-        e = take(*p, &ptr, bytes);
+        if (device_wait()) free_pending(p);
+        (void)cudaStreamSynchronize(p.stream);
+        (void)cudaMemPoolTrimTo(p.pool, 0);
+        e = take(p, &ptr, bytes);
     }
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
@@ -125,13 +164,15 @@ void *device_alloc(size_t bytes, int *device) {
     return ptr;
 }
 
-void device_free(void *ptr, int device) noexcept {
+void device_free(void *ptr, int device, uint64_t context) noexcept {
     if (!ptr) return;
     int previous = device;
     (void)cudaGetDevice(&previous);
     if (previous != device) (void)cudaSetDevice(device);
-    Pool *p = pool_of(device);
-    if (p && p->error == cudaSuccess) {
+    cudaError_t e;
+    // memory of a context that was reset is gone with it
+    Pool *p = context_number() == context ? pool_of(device, context, &e) : nullptr;
+    if (p) {
         bool freed = false;
         if (t_scope) {
             freed = cudaFreeAsync(ptr, t_scope->stream) == cudaSuccess;

@@ -29,8 +29,8 @@ void check_cuda(cudaError_t err, const char *what);
 // lives on a thread, the thread's allocations and frees are ordered on its
 // stream; outside one, an allocation is complete on return and a free waits for
 // the device first.
-void *device_alloc(size_t bytes, int *device);
-void device_free(void *ptr, int device) noexcept;
+void *device_alloc(size_t bytes, int *device, uint64_t *context);
+void device_free(void *ptr, int device, uint64_t context) noexcept;
 // Waits for all work of the current device, as cudaFree does; false where a stream
 // capture forbids it.
 bool device_wait() noexcept;
@@ -52,10 +52,11 @@ struct DeviceArray {
     T *ptr = nullptr;
     size_t count = 0;
     int device = 0;
+    uint64_t context = 0;  // the CUDA context it belongs to (dg_alloc.cu)
     DeviceArray() = default;
     DeviceArray(const DeviceArray &) = delete;
     DeviceArray &operator=(const DeviceArray &) = delete;
-    DeviceArray(DeviceArray &&o) noexcept : ptr(o.ptr), count(o.count), device(o.device) {
+    DeviceArray(DeviceArray &&o) noexcept : ptr(o.ptr), count(o.count), device(o.device), context(o.context) {
         o.ptr = nullptr;
         o.count = 0;
     }
@@ -65,6 +66,7 @@ struct DeviceArray {
             ptr = o.ptr;
             count = o.count;
             device = o.device;
+            context = o.context;
             o.ptr = nullptr;
             o.count = 0;
         }
@@ -74,11 +76,11 @@ struct DeviceArray {
     void alloc(size_t n) {
         release();
         if (n == 0) n = 1;
-        ptr = static_cast<T *>(device_alloc(n * sizeof(T), &device));
+        ptr = static_cast<T *>(device_alloc(n * sizeof(T), &device, &context));
         count = n;
     }
     void release() {
-        if (ptr) device_free(ptr, device);
+        if (ptr) device_free(ptr, device, context);
         ptr = nullptr;
         count = 0;
     }
