@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
                         const bool end = sizeof(P) == 2 && in[i] && (px[i] == 0 || px[i] + 1 == a.n_pixels);
                         ends = ends || end;
                         in[i] = in[i] && !end;
-                        px[i] *= unsigned(sizeof(P));
+                        if constexpr (sizeof(P) == 2) px[i] *= 2u;  // in bytes
                     }
                     const char *next = src;  // the next frame to copy
                     auto issue = [&](int f, int half) {
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
                             for (int i = 0; i < KSTEP; ++i) {
                                 const unsigned d = raw_a + unsigned((half * SB + g * KSTEP + i) * 32) * unsigned(sizeof(W));
                                 if constexpr (sizeof(P) == 8) {
-                                    if (in[i]) cp_async8_s(d, fs + px[i]);
+                                    if (in[i]) cp_async8_s(d, fs + size_t(px[i]) * 8u);
                                 } else {
                                     if (in[i]) cp_async4_s(d, fs + ((px[i] + low) & ~3u));
                                 }
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
                             if (lane + 32 * i < d && !in[i])
                                 for (int f = 0; f < nf; ++f)
                                     rows[f * STRIDE + 32 * i] = load_px<P>(
-                                        fbase + int64_t(f) * a.n_pixels + px[i] / unsigned(sizeof(P)), 0u);
+                                        fbase + int64_t(f) * a.n_pixels + px[i] / 2u, 0u);
                     }
                 }
                 if constexpr (MODE == kRaw) {
