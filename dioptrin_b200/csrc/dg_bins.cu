@@ -1150,11 +1150,15 @@ void lay_out_bin_tiles(const int64_t *rp, const int32_t *col, int64_t nb, BinLay
     for (const BinTile &T : tiles) all_chunks += int64_t(T.chunks.size());
     const int piece = int(std::clamp<int64_t>(all_chunks / 350, kBtPieceMin, kBtPieceMax));
     // Neighbouring tiles whose pieces are claimed one after the other: they walk the
-    // same rows at the same time and share the sectors at their common edges (Eiger-4M
-    // batch of 256 with the spread: by size alone 1846 us, 2 tiles 1776, 4 tiles 1738, 5
-    // tiles 1749). Frames of few pieces need an even finish more (Pilatus 1M, 50 frames:
-    // 2 tiles 109 us, 4 tiles 113, 5 tiles 129; 256 frames: 405, 412, 410).
-    const int64_t near = piece == kBtPieceMax ? 4 : 2;
+    // same rows at the same time and share the sectors at their common edges. Four
+    // tiles where a table has more chunks than the shortest pieces take (22,750), two
+    // where an even finish of few pieces counts more. us with two and with four:
+    // Eiger-4M (27,619 chunks), 256 frames with the spread 1757 and 1731, with errors
+    // 1526 and 1458, 64 frames with the spread 474 and 466; 2600 x 2500 pixels (40,128),
+    // 128 frames with the spread 1325 and 1303; Eiger-9M (62,558), 128 frames with
+    // errors 1697 and 1686, 192 with the spread 2906 and 2926; Pilatus 1M (6,639), 256
+    // frames 405 and 415, 50 frames 117 and 119.
+    const int64_t near = piece > kBtPieceMin ? 4 : 2;
     std::vector<std::vector<BinPiece>> &cut = out.cut;
     cut.resize(static_cast<size_t>(n_items));
     std::atomic<bool> any_cut{false};
