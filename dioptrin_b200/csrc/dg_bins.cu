@@ -56,8 +56,11 @@
 #include <algorithm>
 #include <atomic>
 #include <climits>
+#include <exception>
 #include <map>
 #include <memory>
+#include <mutex>
+#include <system_error>
 #include <thread>
 
 #include "dg_gather_common.cuh"
@@ -1018,18 +1021,34 @@ struct BinLayout {
     int32_t n_slots = 0;
 };
 
-// fn(0) .. fn(count - 1) over host threads.
+// fn(0) .. fn(count - 1) over host threads, the caller's among them. The first
+// exception is thrown on the caller's thread once all have stopped; where no more
+// threads can be made, those that there are do the work.
 template <class Fn>
 void parallel(int64_t count, Fn &&fn) {
     const int nt = int(std::min<int64_t>(
         count, std::max(1u, std::min(16u, std::thread::hardware_concurrency()))));
-    std::vector<std::thread> pool;
     std::atomic<int64_t> next{0};
-    for (int t = 0; t < nt; ++t)
-        pool.emplace_back([&]() {
+    std::mutex mu;
+    std::exception_ptr error;
+    auto run = [&]() {
+        try {
             for (int64_t i; (i = next.fetch_add(1)) < count;) fn(i);
-        });
+        } catch (...) {
+            next = count;
+            std::lock_guard<std::mutex> lock(mu);
+            if (!error) error = std::current_exception();
+        }
+    };
+    std::vector<std::thread> pool;
+    pool.reserve(size_t(std::max(nt, 1)));
+    try {
+        while (int(pool.size()) + 1 < nt) pool.emplace_back(run);
+    } catch (const std::system_error &) {
+    }
+    run();
     for (auto &th : pool) th.join();
+    if (error) std::rethrow_exception(error);
 }
 
 // Bin tiles (k_gather_bins) at plan time, on the host: for every run of
@@ -1053,11 +1072,13 @@ void lay_out_bin_tiles(const int64_t *rp, const int32_t *col, int64_t nb, BinLay
         // pixel << 32 | row << 27 | position in row; each row is sorted
         // already, so four rounds of pairwise merges order the tile.
         const int64_t n_e = rp[r1] - rp[r0];
+        for (int64_t r = r0; r < r1; ++r)
+            if (rp[r + 1] - rp[r] >= (int64_t(1) << 27))
+                fail(DG_UNSUPPORTED, "a bin too large for bin tiles");
         std::vector<uint64_t> ka(static_cast<size_t>(n_e)), kb(static_cast<size_t>(n_e));
         std::vector<int64_t> bounds(static_cast<size_t>(kBtRows) + 1, 0);
         for (int j = 0; j < nr; ++j) {
             const int64_t b = rp[r0 + j], e = rp[r0 + j + 1];
-            if (e - b >= (int64_t(1) << 27)) fail(DG_UNSUPPORTED, "a bin too large for bin tiles");
             uint64_t *o = ka.data() + (b - rp[r0]);
             for (int64_t k = b; k < e; ++k)
                 o[k - b] = (uint64_t(uint32_t(col[k])) << 32) | (uint64_t(j) << 27) |
