@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(kThreads)
 // ahead (the registers cost a CTA per SM).
 constexpr int kRowsLong = 512;
 constexpr int kRowsTiny = 64;  // rows of at most this many entries take 8 lanes
-constexpr int kRowsU = 4;  // entries in flight per thread
+constexpr int kRowsU = 4;  // entries in flight per thread (RowsForm takes fewer in one form)
 constexpr int kRowsThreads = 256;
 
 // Butterfly sum over the 32 lanes: every lane ends with the same value (IEEE
@@ -515,7 +515,7 @@ __device__ __forceinline__ void rows_origin(const QueuePlan &qp, const int4 rec,
 
 // This thread's sums of entries e0 + li, e0 + li + nl, ... < e1 of a row (rec:
 // {row, first entry, end, origin}) in frames f0 .. f0 + F - 1.
-template <int MODE, typename P, int F>
+template <int MODE, typename P, int F, int U = kRowsU>
 __device__ __forceinline__ void rows_sum(const QueuePlan &qp, const int4 rec, int e0, int e1, int li,
                                          int nl, int f0, const double (&o)[F],
                                          double (&acc)[F][NAcc<MODE, P>::value]) {
@@ -532,14 +532,14 @@ __device__ __forceinline__ void rows_sum(const QueuePlan &qp, const int4 rec, in
     for (int q = 0; q < F; ++q)
 #pragma unroll
         for (int a = 0; a < NA; ++a) acc[q][a] = 0.0;
-    for (int j0 = e0 + li; j0 < e1; j0 += nl * kRowsU) {
+    for (int j0 = e0 + li; j0 < e1; j0 += nl * U) {
         // Loads past the end repeat the last entry with weight 0 and pixel 0: no
         // load waits behind a branch.
-        float cw[kRowsU];
-        [[maybe_unused]] float2 nn[kRowsU];
-        P raw[kRowsU][F];
+        float cw[U];
+        [[maybe_unused]] float2 nn[U];
+        P raw[U][F];
 #pragma unroll
-        for (int u = 0; u < kRowsU; ++u) {
+        for (int u = 0; u < U; ++u) {
             const int j = j0 + nl * u;
             const int2 en = entry[min(j, e1 - 1)];
             const uint32_t col = uint32_t(en.x);
@@ -549,7 +549,7 @@ __device__ __forceinline__ void rows_sum(const QueuePlan &qp, const int4 rec, in
             for (int q = 0; q < F; ++q) raw[u][q] = __ldg(fr[q] + col);
         }
 #pragma unroll
-        for (int u = 0; u < kRowsU; ++u) {
+        for (int u = 0; u < U; ++u) {
             if (is_float_px<P>() && j0 + nl * u >= e1) {
 #pragma unroll
                 for (int q = 0; q < F; ++q) raw[u][q] = P(0);
@@ -601,7 +601,7 @@ __device__ __forceinline__ int2 rows_eighth(const int4 rec, int w) {
 
 // One row-warp item of a plan's batch (q.item[k]); every thread of the CTA
 // calls it. F frames, one pass over the entries.
-template <int MODE, typename P, int F>
+template <int MODE, typename P, int F, int U = kRowsU>
 __device__ __forceinline__ void rows_item(const QueuePlan &qp, int k, int fb, RowsRed &s_red) {
     constexpr int NA = NAcc<MODE, P>::value;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -611,7 +611,7 @@ __device__ __forceinline__ void rows_item(const QueuePlan &qp, int k, int fb, Ro
         const int4 rec = qp.rows[k];
         const int2 e = rows_eighth(rec, warp);
         rows_origin<MODE, P, F>(qp, rec, f0, o);
-        rows_sum<MODE, P, F>(qp, rec, e.x, e.y, lane, 32, f0, o, acc);
+        rows_sum<MODE, P, F, U>(qp, rec, e.x, e.y, lane, 32, f0, o, acc);
 #pragma unroll
         for (int q = 0; q < F; ++q)
 #pragma unroll
@@ -644,7 +644,7 @@ __device__ __forceinline__ void rows_item(const QueuePlan &qp, int k, int fb, Ro
     const int4 rec = qp.rows[live ? at : first];
     const int li = tiny ? lane & 7 : lane;
     rows_origin<MODE, P, F>(qp, rec, f0, o);
-    rows_sum<MODE, P, F>(qp, rec, rec.y, live ? rec.z : rec.y, li, tiny ? 8 : 32, f0, o, acc);
+    rows_sum<MODE, P, F, U>(qp, rec, rec.y, live ? rec.z : rec.y, li, tiny ? 8 : 32, f0, o, acc);
 #pragma unroll
     for (int q = 0; q < F; ++q)
 #pragma unroll
@@ -696,25 +696,47 @@ __global__ void k_row_origins(int4 *__restrict__ rows, const int32_t *__restrict
 }
 
 // Lane mapping 10 for one plan's batch: one CTA per (item, frame block).
-// Resident CTAs per SM the compiler must allow for: what hides the loads' latency
-// is warps. One frame without the spread, 8 (32 registers) against 6: Eiger-4M cake
-// 59.4 and 67.6 us; the others 4 (64 registers) against what the compiler takes:
-// two frames with the spread 69.6 and 75.9, 64 Eiger-9M frames 708 and 738. Four
-// frames with the spread would spill (186 against 125). A launch that leaves SMs
-// with few CTAs anyway (small, one frame) takes the registers that shorten it.
-template <int MODE>
-constexpr int rows_min_ctas(int f, bool small) {
-    return small ? 1 : MODE != kSpread ? (f == 1 ? 8 : 4) : f == 4 ? 1 : 4;
+// Forms of the kernel without the spread: what hides the loads' latency is loads per
+// thread where a launch leaves SMs with few CTAs, and CTAs per SM where it does not.
+// The sums do not depend on the form.
+enum RowsForm {
+    kRowsFew,    // few CTAs per SM (launch_rows): the registers of all its loads
+    kRowsMany,
+    kRowsShort,  // many CTAs, most of them of rows of at most kRowsLong entries
+};
+// Resident CTAs per SM the compiler must allow for. us, graph-timed, Eiger-4M u32:
+// four frames with errors, 3000 bins, 3 CTAs per SM 95.0, 4 100.7, unbounded 109.3;
+// 1000 bins, intensities, 3 39.5, 4 36.3; two frames with errors, 3000 bins, 3 entries
+// in flight and 4 CTAs 53.8, 4 and 4 62.4, 4 and 3 57.8; two float frames with the spread,
+// 3000 bins, 3 CTAs 106, 4 (spilled) 128; an Eiger-4M cake, two frames of u16
+// intensities, 6 CTAs 19.2, 4 21.7. One frame without the spread, 8 CTAs against 6:
+// Eiger-4M cake 59.4 and 67.6. Four frames with the spread would spill (186 against
+// 125 with 4 CTAs).
+template <int MODE, typename P>
+constexpr int rows_min_ctas(int f, RowsForm form) {
+    if (MODE == kSpread) return f == 4 ? 1 : f == 2 && is_float_px<P>() ? 3 : 4;
+    if (form == kRowsFew) return f == 1 ? 4 : 3;
+    if (f == 1) return 8;
+    if (f == 2) return form == kRowsShort ? 6 : 4;
+    return MODE == kErrors && sizeof(P) >= 4 ? 3 : 4;
 }
-template <int MODE, typename P, int F, bool SMALL = false>
-__global__ void __launch_bounds__(kRowsThreads, rows_min_ctas<MODE>(F, SMALL)) k_rows(const QueuePlan q, const int groups) {
+// Entries in flight per thread.
+template <int MODE, typename P>
+constexpr int rows_loads(int f, RowsForm form) {
+    return MODE != kSpread && f == 2 && form == kRowsMany && !(MODE == kErrors && is_float_px<P>())
+               ? 3
+               : kRowsU;
+}
+template <int MODE, typename P, int F, RowsForm FORM>
+__global__ void __launch_bounds__(kRowsThreads, rows_min_ctas<MODE, P>(F, FORM))
+    k_rows(const QueuePlan q, const int groups) {
     __shared__ RowsRed s_red;
     int k = blockIdx.x;
-    if constexpr (F == 4) {
+    if constexpr (F == 4 && FORM == kRowsMany) {
         if (k < groups) return rows_group<MODE, P, F>(q, k, blockIdx.y, s_red);
         if (groups) k += q.n_long - groups;
     }
-    rows_item<MODE, P, F>(q, k, blockIdx.y, s_red);
+    rows_item<MODE, P, F, rows_loads<MODE, P>(F, FORM)>(q, k, blockIdx.y, s_red);
 }
 
 // Frames per pass (and per frame block) of a row-warp launch of nf frames.
@@ -1636,24 +1658,51 @@ template <int MODE, typename P>
 void launch_rows(const GatherTable &t, const P *fp, int64_t n_pixels, int nf, double *oi,
                  double *os, double *od, cudaStream_t s) {
     const QueuePlan q = queue_plan(t, fp, n_pixels, nf, oi, os, od);
-    // Long rows in groups of eight (rows_group) once those fill the chip: a group is
-    // a serial walk of eight rows. Eiger-4M with the spread, 235 groups, us, a CTA
-    // per row against groups: 4 frames 122 / 170, 16 frames 442 / 352, 64 frames 1721
-    // / 1347; Eiger-9M intensities, 124 groups: 8 frames 93 / 166, 16 frames 182 /
-    // 190, 32 frames 358 / 337, 64 frames 709 / 596. Four per SM is where they cross.
+    // Long rows in groups of eight (rows_group): a group is a serial walk of eight
+    // rows, so it pays once there are several groups per SM, the more the thicker
+    // the rings (longer and fewer rows): a row then shares fewer sectors with its
+    // neighbours. us, a CTA per row against groups: Eiger-9M u16, 1000 bins,
+    // intensities, 32 / 64 frames (7 and 13 groups per SM, line at 11) 331 / 334 and
+    // 653 / 594, with errors, 64 frames (line at 14) 677 / 764; 2000 bins with errors,
+    // 16 / 24 frames (7 and 10, line at 6) 286 / 295 and 422 / 371; Eiger-4M u32 with
+    // the spread, 1000 bins, 24 / 32 / 64 frames (5, 6 and 13, line at 6) 402 / 425, 532
+    // / 532 and 1050 / 975, 2000 bins, 8 frames (3, line at 4) 228 / 177. A row much
+    // longer than the others would hold its warp long after they are done.
     int groups = (q.n_long + kRowsWarps - 1) / kRowsWarps;
-    if (rows_pass_frames(nf) < 4 || int64_t(groups) * q.frame_blocks < 4 * sm_count()) groups = 0;
-    const dim3 grid(unsigned(q.n_items - (groups ? q.n_long - groups : 0)), unsigned(q.frame_blocks));
-    switch (rows_pass_frames(nf)) {
-    case 1:
-        if (q.n_items <= 2 * sm_count())
-            k_rows<MODE, P, 1, true><<<grid, kRowsThreads, 0, s>>>(q, groups);
-        else
-            k_rows<MODE, P, 1><<<grid, kRowsThreads, 0, s>>>(q, groups);
-        break;
-    case 2: k_rows<MODE, P, 2><<<grid, kRowsThreads, 0, s>>>(q, groups); break;
-    default: k_rows<MODE, P, 4><<<grid, kRowsThreads, 0, s>>>(q, groups); break;
+    if (rows_pass_frames(nf) < 4 || q.n_long == 0) {
+        groups = 0;
+    } else {
+        const double mean = double(t.rw_long_entries) / q.n_long;
+        const double per_sm = double(groups) * q.frame_blocks / sm_count();
+        const double slope = MODE == kSpread ? 0.5 : MODE == kErrors ? 1.0 : 0.75;
+        if (per_sm < 2.0 + slope * mean / q.n_long || t.rw_longest > 4.0 * mean) groups = 0;
     }
+    const dim3 grid(unsigned(q.n_items - (groups ? q.n_long - groups : 0)), unsigned(q.frame_blocks));
+    auto go = [&](auto frames, auto form) {
+        k_rows<MODE, P, decltype(frames)::value, decltype(form)::value>
+            <<<grid, kRowsThreads, 0, s>>>(q, groups);
+    };
+    using Few = std::integral_constant<RowsForm, kRowsFew>;
+    using Many = std::integral_constant<RowsForm, kRowsMany>;
+    using Short = std::integral_constant<RowsForm, kRowsShort>;
+    const int f = rows_pass_frames(nf);
+    // Where the lines between the forms lie (us, graph-timed, few against many): one
+    // frame, u16 with errors, 6 CTAs per SM 11.2 / 12.4 and 13.9 / 16.0, 11 per SM 11.5 /
+    // 10.4, 38 per SM (a cake) 19.3 / 16.4; two frames, u32 intensities, 2 per SM 17.9 /
+    // 19.4, 7 per SM 23.8 / 22.0; four, 2 per SM 46.1 / 53.4, 7 per SM 39.5 / 36.3. Against
+    // the kernel with predicated loads and no forms, two frames at 5 to 7 CTAs per SM
+    // are up to 1.2 us (13 %) slower, all other forms as fast or faster.
+    const bool few = MODE != kSpread && !groups && int64_t(grid.x) * grid.y <= (f == 1 ? 8 : 3) * sm_count();
+    auto either = [&](auto frames) {
+        if constexpr (MODE != kSpread)
+            if (few) return go(frames, Few{});
+        if constexpr (MODE != kSpread && decltype(frames)::value == 2)
+            if (4 * q.n_long < 3 * q.n_items) return go(frames, Short{});
+        go(frames, Many{});
+    };
+    if (f == 1) either(std::integral_constant<int, 1>{});
+    else if (f == 2) either(std::integral_constant<int, 2>{});
+    else either(std::integral_constant<int, 4>{});
     DG_CUDA(cudaGetLastError());
 }
 
@@ -1984,6 +2033,10 @@ void make_gather_table(const DeviceCsr &table, const double *d_norm, int32_t dim
             return int32_t(rw_rows.size());
         };
         out.rw_long = take(kRowsLong, INT64_MAX);
+        for (const int4 &r : rw_rows) {
+            out.rw_long_entries += r.z - r.y;
+            out.rw_longest = std::max<int64_t>(out.rw_longest, r.z - r.y);
+        }
         // neighbours stay together in groups of kRowsWarps, the longest rows first
         std::vector<int4> by_row(rw_rows);
         std::vector<std::pair<int64_t, size_t>> groups;

@@ -342,6 +342,7 @@ struct GatherTable {
     // each), then to rw_tiny the rows of more than kRowsTiny (eight per CTA, a warp
     // each), then the others (32 per CTA, eight lanes each); rw_n_items CTAs.
     int32_t rw_long = 0, rw_tiny = 0;
+    int64_t rw_long_entries = 0, rw_longest = 0;  // of the long rows, and of the longest
     int32_t rw_n_items = 0;
     // Per pixel (frame storage order) its norm n as an FP32 pair {n, n - n32},
     // {0, 0} where n is not finite or not positive: the row warps' spread
