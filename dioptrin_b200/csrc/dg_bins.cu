@@ -14,8 +14,9 @@
 // Producers and consumers. The kernel is persistent, one CTA per SM, and runs
 // its work items' chunks as one stream through a ring of BUFS shared-memory
 // buffers. Producer warps stage a chunk: its pixels (4-byte pixel types by
-// 4-byte cp.async, one instruction per 32 pixels of a frame; 2- and 8-byte ones
-// by cp.async into a ring of the warp's own, then converted to FP32 and stored)
+// 4-byte cp.async, one instruction per 32 pixels of a frame; 2-byte ones alike, as
+// the words that hold them; 8-byte ones by cp.async into a ring of the warp's own,
+// then converted to FP32 and stored)
 // into frame rows STRIDE words apart (odd, so the 32 lanes reading one pixel of
 // their frames hit 32 banks), and by one thread's bulk copies its pair records
 // and row offsets. Consumer warps only sum. "full" barriers count the producers' copies, "empty" barriers the
@@ -37,6 +38,13 @@
 // one piece; a piece leaves FP64 partial sums, and the CTA that finishes a
 // tile's last piece adds them in piece order. A finished tile is normalised and
 // written through shared memory, so that a frame's ROWS results are one run.
+//
+// 2-byte pixels went through the ring of the 8-byte ones, two instructions more per
+// pixel for few warps and a memory latency per batch of frames; now the sums take
+// their half of the word. Mapping 8, u16, us, through the ring and now: Pilatus 1M, 64
+// / 256 frames with errors 212 / 665 and 155 / 482, with the spread 309 / 980 and 205 /
+// 654; Eiger-4M, 256 frames with the spread 3616 and 2301, per-frame masks, 64 frames
+// 1376 and 943.
 //
 // What bounds it: the load-store unit. A 4-byte cp.async of 32 pixels that lie in
 // two or three short runs holds it for about 11 cycles (two per 32-byte sector);
@@ -123,22 +131,17 @@ struct BtCfg {
     static constexpr int threads() {
         return (ROWS + producers<MODE, P>()) * 32;
     }
-    // Converted pixel types: a producer copies kSteps pixels per lane at a time
-    // (kRawFrames frames) into its own ring of two such batches.
+    // 8-byte pixels: a producer copies batches of raw_frames frames into a ring of its
+    // own of two batches.
     static constexpr int kLaneSlots = (DCAP + 31) / 32;
-    template <typename P>
-    static constexpr int raw_frames() {
-        return kLaneSlots > 6 ? 1 : sizeof(P) == 8 ? 2 : 4;
-    }
+    static constexpr int kRawFrames = kLaneSlots > 6 ? 1 : 2;
     template <int MODE, typename P>
     static constexpr size_t raw_bytes() {
-        return sizeof(P) == 4 ? 0
-                              : size_t(producers<MODE, P>()) * 2 * raw_frames<P>() * kLaneSlots * 32 *
-                                    (sizeof(P) == 8 ? 8 : 4);
+        return sizeof(P) == 8 ? size_t(producers<MODE, P>()) * 2 * kRawFrames * kLaneSlots * 32 * 8 : 0;
     }
     template <typename P>
     static constexpr int bufs() {  // the ring of mapping 7 takes the third buffer's place
-        return sizeof(P) == 4 || F2 == 2 ? BUFS : 2;
+        return sizeof(P) != 8 || F2 == 2 ? BUFS : 2;
     }
     // A buffer: frame rows, pairs A, then B (spread, masks), C (spread), the
     // record's head, then a word of frame bits per slot (masks); every part
@@ -260,6 +263,11 @@ __device__ __forceinline__ uint32_t lds32_at(unsigned a) {
     asm volatile("ld.shared.b32 %0, [%1+%2];\n" : "=r"(v) : "r"(a), "n"(OFF));
     return v;
 }
+__device__ __forceinline__ uint2 lds64(unsigned a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
 
 // ------------------------------------------------------------- the kernel
 
@@ -298,9 +306,10 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
     constexpr bool SPREAD = MODE == kSpread;
     constexpr bool WIDE = SPREAD || MODE == kRaw;  // pairs B
     constexpr bool FLOAT_SPREAD = SPREAD && is_float_px<P>();
-    constexpr bool COPIES = sizeof(P) == 4;                  // pixels by cp.async
+    constexpr bool HALF = sizeof(P) == 2;                    // pixels as the words that hold them
+    constexpr bool COPIES = sizeof(P) == 4 || HALF;          // pixels by cp.async
     constexpr bool ASYNC = COPIES || MODE == kRaw;           // some cp.async per chunk
-    constexpr bool STORES = !COPIES;                         // plain stores
+    constexpr bool STORES = sizeof(P) != 4;                  // plain stores (2-byte: of a frame's ends)
     constexpr int F2 = CFG::kF2, STRIDE = CFG::kStride, DCAP = CFG::kDCap, PCAP = CFG::kPCap;
     constexpr int U2 = bt_step<MODE, P, CFG>();
     constexpr int NW = CFG::kRows, NP = CFG::template producers<MODE, P>(), NB = CFG::template bufs<P>();
@@ -351,9 +360,7 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
 
     if (warp >= NW) {
         // ------------------------------------------------------- producers
-        constexpr int FPW = CFG::kFrames / NP;         // frames per producer warp
         constexpr int KSTEP = (DCAP + 31) / 32;
-        static_assert(CFG::kFrames % NP == 0, "producers share the frames evenly");
         const int pw = warp - NW;
         const bool claims = pw == 0 && lane == 0;
         int claim = claims ? atomicAdd(a.counter, 1) : 0;
@@ -391,9 +398,13 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
                 break;
             }
             const int4 it = a.items[item];
-            const int f0 = group * CFG::kFrames + pw * FPW;
-            const int nf = min(FPW, a.n_frames - f0);  // this warp's frames, may be <= 0
-            const P *fbase = frames + int64_t(f0) * a.n_pixels;
+            // this warp's frames of the group, from fw on (nf may be <= 0): even shares,
+            // but for 4-byte pixels fixed ones (with even ones a Pilatus batch of 256,
+            // whose shares are the same, took 417 us against 399)
+            const int gf = min(CFG::kFrames, a.n_frames - group * CFG::kFrames);
+            const int per = sizeof(P) == 4 ? CFG::kFrames / NP : (gf + NP - 1) / NP, fw = pw * per;
+            const int nf = min(per, gf - fw);
+            const P *fbase = frames + int64_t(group * CFG::kFrames + fw) * a.n_pixels;
             const int32_t *rec = a.meta + int64_t(it.z) * MW;
             // the next chunk's record is read while this one's copies are issued
             int n_px = rec[0], n_pr = rec[1], first = rec[2];
@@ -433,9 +444,43 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
                 bool in[KSTEP];
 #pragma unroll
                 for (int i = 0; i < KSTEP; ++i) in[i] = lane + 32 * i < d;
-                unsigned dst = buf + unsigned(pw * FPW * STRIDE + lane) * 4u;
+                unsigned dst = buf + unsigned(fw * STRIDE + lane) * 4u;
                 const char *src = reinterpret_cast<const char *>(fbase);
-                if constexpr (COPIES) {
+                if constexpr (HALF) {
+                    // 2-byte pixels as the aligned words that hold them, and the sums take
+                    // their half; at the ends of a frame, where that word may reach outside
+                    // the array, a word made of the pixel.
+                    bool ends = false;
+#pragma unroll
+                    for (int i = 0; i < KSTEP; ++i) {
+                        const bool end = in[i] && (px[i] == 0 || px[i] + 1 == a.n_pixels);
+                        ends = ends || end;
+                        in[i] = in[i] && !end;
+                        px[i] *= 2u;
+                    }
+                    if (__any_sync(0xffffffffu, ends)) {
+                        uint32_t *rows = reinterpret_cast<uint32_t *>(smem + b * BUF) + fw * STRIDE + lane;
+#pragma unroll
+                        for (int i = 0; i < KSTEP; ++i)
+                            if (lane + 32 * i < d && !in[i])
+                                for (int f = 0; f < nf; ++f) {
+                                    const P *at = fbase + int64_t(f) * a.n_pixels + px[i] / 2u;
+                                    rows[f * STRIDE + 32 * i] =
+                                        uint32_t(__ldg(at)) << (unsigned(reinterpret_cast<uintptr_t>(at)) & 2u) * 8u;
+                                }
+                    }
+                    constexpr int UNROLL = CFG::template copy_unroll<MODE>();
+#pragma unroll UNROLL
+                    for (int f = 0; f < nf; ++f) {
+                        const unsigned low = unsigned(reinterpret_cast<uintptr_t>(src)) & 2u;
+                        const char *fs = src - low;
+#pragma unroll
+                        for (int i = 0; i < KSTEP; ++i)
+                            if (in[i]) cp_async4_s(dst + 128u * i, fs + ((px[i] + low) & ~3u));
+                        dst += STRIDE * 4u;
+                        src += a.n_pixels * 2;
+                    }
+                } else if constexpr (COPIES) {
 #pragma unroll
                     for (int i = 0; i < KSTEP; ++i) px[i] *= 4u;
                     constexpr int UNROLL = CFG::template copy_unroll<MODE>();
@@ -448,48 +493,28 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
                         src += a.n_pixels * 4;
                     }
                 } else {
-                    // Converted pixels: FB frames' copies into half of this warp's
-                    // ring while the other half is converted and stored. A lane reads
-                    // back what it copied itself. 2-byte pixels come as the aligned
-                    // word that holds them, except at the ends of a frame, where that
-                    // word may reach outside the array.
-                    using W = typename std::conditional<sizeof(P) == 8, P, uint32_t>::type;
-                    constexpr int FB = CFG::template raw_frames<P>(), SB = FB * KSTEP;
-                    W *raw = reinterpret_cast<W *>(smem + CFG::template raw_off<MODE, P>()) +
+                    // 8-byte pixels: FB frames' copies into half of this warp's ring
+                    // while the other half is converted and stored. A lane reads back
+                    // what it copied itself.
+                    constexpr int FB = CFG::kRawFrames, SB = FB * KSTEP;
+                    P *raw = reinterpret_cast<P *>(smem + CFG::template raw_off<MODE, P>()) +
                              pw * 2 * SB * 32 + lane;
                     const unsigned raw_a = smem_addr(raw);
-                    bool ends = false;
-#pragma unroll
-                    for (int i = 0; i < KSTEP; ++i) {
-                        const bool end = sizeof(P) == 2 && in[i] && (px[i] == 0 || px[i] + 1 == a.n_pixels);
-                        ends = ends || end;
-                        in[i] = in[i] && !end;
-                        if constexpr (sizeof(P) == 2) px[i] *= 2u;  // in bytes
-                    }
                     const char *next = src;  // the next frame to copy
                     auto issue = [&](int f, int half) {
 #pragma unroll
                         for (int g = 0; g < FB; ++g) {
                             if (f + g >= nf) break;
-                            // the frame's start on a word boundary, and how far past it
-                            const unsigned low = sizeof(P) == 2 ? unsigned(reinterpret_cast<uintptr_t>(next)) & 2u : 0u;
-                            const char *fs = next - low;
 #pragma unroll
-                            for (int i = 0; i < KSTEP; ++i) {
-                                const unsigned d = raw_a + unsigned((half * SB + g * KSTEP + i) * 32) * unsigned(sizeof(W));
-                                if constexpr (sizeof(P) == 8) {
-                                    if (in[i]) cp_async8_s(d, fs + size_t(px[i]) * 8u);
-                                } else {
-                                    if (in[i]) cp_async4_s(d, fs + ((px[i] + low) & ~3u));
-                                }
-                            }
-                            next += a.n_pixels * int64_t(sizeof(P));
+                            for (int i = 0; i < KSTEP; ++i)
+                                if (in[i])
+                                    cp_async8_s(raw_a + unsigned((half * SB + g * KSTEP + i) * 32) * 8u,
+                                                next + size_t(px[i]) * 8u);
+                            next += a.n_pixels * 8;
                         }
                         asm volatile("cp.async.commit_group;\n" ::: "memory");
                     };
-                    const unsigned low0 = unsigned(reinterpret_cast<uintptr_t>(fbase)) & 2u;
-                    const unsigned low_step = unsigned(a.n_pixels & 1) * 2u;
-                    float *rows = reinterpret_cast<float *>(smem + b * BUF) + pw * FPW * STRIDE + lane;
+                    float *rows = reinterpret_cast<float *>(smem + b * BUF) + fw * STRIDE + lane;
                     issue(0, 0);
                     int half = 0;
                     for (int f = 0; f < nf; f += FB) {
@@ -498,27 +523,13 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
 #pragma unroll
                         for (int g = 0; g < FB; ++g) {
                             if (f + g >= nf) break;
-                            [[maybe_unused]] const unsigned low = low0 + unsigned(f + g) * low_step;
 #pragma unroll
                             for (int i = 0; i < KSTEP; ++i) {
-                                const W w = raw[(half * SB + g * KSTEP + i) * 32];
-                                float v;
-                                if constexpr (sizeof(P) == 8)
-                                    v = __double2float_rn(w);
-                                else
-                                    v = float((px[i] + low) & 2u ? w >> 16 : w & 0xffffu);
+                                const float v = __double2float_rn(raw[(half * SB + g * KSTEP + i) * 32]);
                                 if (in[i]) rows[(f + g) * STRIDE + 32 * i] = v;
                             }
                         }
                         half ^= 1;
-                    }
-                    if (__any_sync(0xffffffffu, ends)) {
-#pragma unroll
-                        for (int i = 0; i < KSTEP; ++i)
-                            if (lane + 32 * i < d && !in[i])
-                                for (int f = 0; f < nf; ++f)
-                                    rows[f * STRIDE + 32 * i] = load_px<P>(
-                                        fbase + int64_t(f) * a.n_pixels + px[i] / 2u, 0u);
                     }
                 }
                 if constexpr (MODE == kRaw) {
@@ -598,6 +609,15 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
             ex_n[h] = 0;
         }
         int since = 0;
+        // 2-byte pixels: the bytes of a word that hold an even pixel of this lane's frames
+        // (alike for frames 32 apart), and the step to an odd one's, below the upper
+        // bytes of 2^23: the float 2^23 + pixel, without a conversion's slow unit.
+        [[maybe_unused]] unsigned sel_even = 0x7610u, sel_odd = 0x22u;
+        if constexpr (HALF)
+            if (reinterpret_cast<uintptr_t>(frames + int64_t(f0 + lane) * a.n_pixels) & 2u) {
+                sel_even = 0x7632u;
+                sel_odd = 0u - 0x22u;
+            }
         // Origin of the spread's shift, per frame of the lane (row_origin).
         f2 norg[F2];
 #pragma unroll
@@ -633,7 +653,7 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
                 const float4 *s_pa = reinterpret_cast<const float4 *>(buf + PAIRS);
                 const float4 *s_pb = s_pa + PCAP;
                 const f2 *s_pc = reinterpret_cast<const f2 *>(buf + PAIRS + PCAP * 32u);
-                [[maybe_unused]] const uint2 *mk = reinterpret_cast<const uint2 *>(buf + MASKS);
+                [[maybe_unused]] const unsigned mk = base + b * BUF + MASKS;
                 [[maybe_unused]] const unsigned my_bit = 1u << lane;
                 auto body = [&](int p, auto unroll) {
                     constexpr int UU = decltype(unroll)::value;
@@ -650,13 +670,22 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
                     float v0[F2][UU], v1[F2][UU];
 #pragma unroll
                     for (int u = 0; u < UU; ++u) {
-                        const unsigned a0 = pxa + 4u * unsigned(__float_as_int(ea[u].x));
-                        const unsigned a1 = pxa + 4u * unsigned(__float_as_int(ea[u].y));
-                        v0[0][u] = staged_value<S>(lds32_at<0>(a0));
-                        v1[0][u] = staged_value<S>(lds32_at<0>(a1));
+                        // slot, and bit 30 (lost in the address): an odd pixel
+                        const unsigned s0 = unsigned(__float_as_int(ea[u].x)), s1 = unsigned(__float_as_int(ea[u].y));
+                        const unsigned a0 = pxa + 4u * s0, a1 = pxa + 4u * s1;
+                        auto value = [&](uint32_t w, [[maybe_unused]] unsigned s) {
+                            if constexpr (HALF)
+                                return __fadd_rn(__uint_as_float(__byte_perm(
+                                                     w, 0x4b000000u, sel_even + (s >> 30) * sel_odd)),
+                                                 -8388608.f);
+                            else
+                                return staged_value<S>(w);
+                        };
+                        v0[0][u] = value(lds32_at<0>(a0), s0);
+                        v1[0][u] = value(lds32_at<0>(a1), s1);
                         if constexpr (F2 == 2) {
-                            v0[F2 - 1][u] = staged_value<S>(lds32_at<128 * STRIDE>(a0));
-                            v1[F2 - 1][u] = staged_value<S>(lds32_at<128 * STRIDE>(a1));
+                            v0[F2 - 1][u] = value(lds32_at<128 * STRIDE>(a0), s0);
+                            v1[F2 - 1][u] = value(lds32_at<128 * STRIDE>(a1), s1);
                         }
                     }
                     if constexpr (MODE == kRaw) {
@@ -666,7 +695,8 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
                         for (int h = 0; h < F2; ++h)
 #pragma unroll
                             for (int u = 0; u < UU; ++u) {
-                                const uint2 w0 = mk[__float_as_int(ea[u].x)], w1 = mk[__float_as_int(ea[u].y)];
+                                const uint2 w0 = lds64(mk + 8u * unsigned(__float_as_int(ea[u].x)));
+                                const uint2 w1 = lds64(mk + 8u * unsigned(__float_as_int(ea[u].y)));
                                 const bool l0 = ((h ? w0.y : w0.x) & my_bit) == 0;
                                 const bool l1 = ((h ? w1.y : w1.x) & my_bit) == 0;
                                 const f2 cc = pk(l0 ? ea[u].z : 0.f, l1 ? ea[u].w : 0.f);
@@ -904,6 +934,13 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
     }
 }
 
+// A pair's slot with bit 30 set where the pixel (as the frame stores it) is odd, which
+// tells the half of a word of 2-byte pixels; the bit is lost in a slot's address (4 or
+// 8 bytes a slot, 32 bits).
+__device__ __forceinline__ float slot_of(int slot, int pixel) {
+    return __int_as_float(slot | (pixel & 1) << 30);
+}
+
 // Bin-tile entry pairs from the plan-time layout: per pair {slot 0, slot 1,
 // entry 0, entry 1} (entry -1: padding, slot = the zero column) to A {slot 0, slot 1,
 // c0, c1} with the table's FP32 weights, AS the same with the spread's
@@ -919,9 +956,11 @@ __global__ void k_bt_fill(const int4 *__restrict__ desc, int64_t n_pairs,
         float c[2] = {0.f, 0.f}, cs[2] = {0.f, 0.f}, n[2] = {1.f, 1.f}, cr[2] = {0.f, 0.f},
               nlo[2] = {0.f, 0.f};
         const int k[2] = {d.z, d.w};
+        int px[2] = {0, 0};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             if (k[h] < 0) continue;
+            px[h] = entry[k[h]].x;
             c[h] = __int_as_float(entry[k[h]].y);
             const float4 es = entry_std[k[h]];
             cs[h] = es.y;
@@ -929,8 +968,9 @@ __global__ void k_bt_fill(const int4 *__restrict__ desc, int64_t n_pairs,
             cr[h] = es.w;
             nlo[h] = entry_nlo[k[h]];
         }
-        pair_a[i] = make_float4(__int_as_float(d.x), __int_as_float(d.y), c[0], c[1]);
-        pair_as[i] = make_float4(__int_as_float(d.x), __int_as_float(d.y), cs[0], cs[1]);
+        const float s0 = slot_of(d.x, px[0]), s1 = slot_of(d.y, px[1]);
+        pair_a[i] = make_float4(s0, s1, c[0], c[1]);
+        pair_as[i] = make_float4(s0, s1, cs[0], cs[1]);
         pair_b[i] = make_float4(n[0], n[1], cr[0], cr[1]);
         pair_c[i] = make_float2(nlo[0], nlo[1]);
     }
@@ -947,14 +987,16 @@ __global__ void k_bt_fill_raw(const int4 *__restrict__ desc, int64_t n_pairs,
         const int4 d = desc[i];
         float w[2] = {0.f, 0.f}, wn[2] = {0.f, 0.f};
         const int k[2] = {d.z, d.w};
+        int px[2] = {0, 0};
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             if (k[h] < 0) continue;
             const float4 e = entry_raw[k[h]];
+            px[h] = __float_as_int(e.x);
             w[h] = e.y;
             wn[h] = e.z;
         }
-        pair_a[i] = make_float4(__int_as_float(d.x), __int_as_float(d.y), w[0], w[1]);
+        pair_a[i] = make_float4(slot_of(d.x, px[0]), slot_of(d.y, px[1]), w[0], w[1]);
         pair_b[i] = make_float4(wn[0], wn[1], 0.f, 0.f);
     }
 }
