@@ -1558,6 +1558,7 @@ bool bin_tiles_fill_gpu(const GatherTable &t, int variant, int64_t n_frames) {
     const int64_t per = variant == 7 ? Bt7::kFrames : Bt8::kFrames;
     const int64_t nf = std::min<int64_t>(n_frames, 256);
     const int64_t ctas = (int64_t(t.n_rows) + rows - 1) / rows * ((nf + per - 1) / per);
+    if (variant == 8 && 2 * nf >= per && bin_tiles_fill_gpu(t, 7, n_frames)) return true;
     return 2 * nf >= per && ctas >= 2 * 148;
 }
 

@@ -481,8 +481,10 @@ void ensure_fl_units(GatherTable &t, const DeviceCsr &table, cudaStream_t s);
 bool bin_tile_wait_failed(const GatherTable &t);
 void check_bin_tile_waits(const GatherTable &t);
 // Whether the autotuner times bin-tile mapping `variant` (7 or 8) for a
-// batch of n_frames: a launch must give every SM at least two CTAs (tiles
-// times frame groups) and fill at least half of each CTA's frames.
+// batch of n_frames: a launch must give every SM at least two tiles (times frame
+// groups; 8 also where 7 does, whose tiles are built anyway: 2-byte pixels of a
+// 1M detector, 4000 bins, 64 frames with the spread, 7 674 us and 8 below 400) and
+// fill at least half of a tile's frames.
 bool bin_tiles_fill_gpu(const GatherTable &t, int variant, int64_t n_frames);
 void prepare_raw(GatherTable &t, const DeviceCsr &table, const double *d_norm, cudaStream_t s);
 void run_gather_raw(GatherTable &t, const void *d_frames, int dtype, int64_t n_pixels,
