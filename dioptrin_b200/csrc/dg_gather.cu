@@ -2372,16 +2372,20 @@ void prepare_raw(GatherTable &t, const DeviceCsr &table, const double *d_norm, c
 
 namespace {
 
+// Per-frame masks on a mapping-8 plan (raw sums S, N, V, C, or the normalised
+// results), and raw sums over the plan mask on a bin-tile plan: the tiles take them.
+bool bin_tiles_take_raw(const GatherTable &t, int mode, bool raw) {
+    return (mode == kRaw ? t.variant == 8 && t.entry_raw.ptr
+                         : raw && gather_variant_needs_tiles(t.variant)) &&
+           t.bt[t.variant - 7].n_items > 0;
+}
+
 template <typename P>
 bool launch_raw(GatherTable &t, const void *frames, int64_t n_pixels, int nf, int mode,
                 const uint8_t *masks, int64_t mask_stride, cudaStream_t s, bool raw, double *o0,
                 double *o1, double *o2, double *o3) {
     const P *fp = static_cast<const P *>(frames);
-    // Per-frame masks on a mapping-8 plan (raw sums S, N, V, C in o0..o3, or the
-    // normalised results in o0, o1), and raw sums over the plan mask on a
-    // bin-tile plan: the tiles take them.
-    if ((mode == kRaw ? t.variant == 8 && t.entry_raw.ptr : raw && gather_variant_needs_tiles(t.variant)) &&
-        t.bt[t.variant - 7].n_items > 0) {
+    if (bin_tiles_take_raw(t, mode, raw)) {
         BinCall c{};
         c.frames = frames;
         c.dtype = dtype_code<P>();
@@ -2419,9 +2423,9 @@ void run_gather_raw(GatherTable &t, const void *d_frames, int dtype, int64_t n_p
     const bool errors = (flags & DG_ERRORS) != 0;
     const int mode = d_masks ? kRaw : errors ? kErrors : kIntensity;
     const int64_t chunk = 256;
-    int64_t rows = std::max<int64_t>(1, t.n_segments);
-    for (int v : {7, 8})
-        if (t.bt[v - 7].n_items > 0) rows = std::max(rows, bin_tile_partials(t, v));
+    // the partial sums of the mapping that runs
+    const int64_t rows = bin_tiles_take_raw(t, mode, raw) ? bin_tile_partials(t, t.variant)
+                                                          : std::max<int64_t>(1, t.n_segments);
     const int64_t need = rows * n_accumulators(mode, dtype == DG_F32 || dtype == DG_F64) *
                          std::min<int64_t>(chunk, (n_frames + 31) / 32 * 32);
     if (t.partial.count < size_t(need)) t.partial.alloc(size_t(need));
