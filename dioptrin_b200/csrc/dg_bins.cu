@@ -16,10 +16,10 @@
 // buffers. Producer warps stage a chunk: its pixels (4-byte pixel types by
 // 4-byte cp.async, one instruction per 32 pixels of a frame; 2-byte ones alike, as
 // the words that hold them; 8-byte ones by cp.async into a ring of the warp's own,
-// then converted to FP32 and stored)
-// into frame rows STRIDE words apart (odd, so the 32 lanes reading one pixel of
-// their frames hit 32 banks), and by one thread's bulk copies its pair records
-// and row offsets. Consumer warps only sum. "full" barriers count the producers' copies, "empty" barriers the
+// then converted to FP32 and stored) into frame rows STRIDE words apart (odd, so
+// the 32 lanes reading one pixel of their frames hit 32 banks), and by one thread's
+// bulk copies its pair records and row offsets. Consumer warps only sum. "full"
+// barriers count the producers' copies, "empty" barriers the
 // consumer warps that have summed the buffer's chunk. When every warp staged a
 // share of each chunk between its sums, 512 threads arrived three times per
 // chunk on barriers in shared memory, the staging addresses took registers of
@@ -341,8 +341,9 @@ __global__ void __launch_bounds__(CFG::template threads<MODE, P>(), 1)
         mbar_init(out_bar, NW);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    // Frame rows start at 0: column DCAP is read by padding pairs and holds 0,
-    // and rows of frames past the batch hold no stray values.
+    // Column DCAP of a frame row is read by padding pairs and stays 0. Rows of frames
+    // past the batch hold zeros or an earlier group's pixels: their sums go nowhere
+    // (results and partial sums are stored for frames below nv alone).
     for (int b = 0; b < NB; ++b) {
         uint32_t *px = reinterpret_cast<uint32_t *>(smem + size_t(b) * BUF);
         for (int j = tid; j < CFG::kFrames * STRIDE; j += NT) px[j] = 0;

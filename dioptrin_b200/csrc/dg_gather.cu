@@ -599,8 +599,9 @@ __device__ __forceinline__ int2 rows_eighth(const int4 rec, int w) {
     return make_int2(rec.y + int(n * w / kRowsWarps), rec.y + int(n * (w + 1) / kRowsWarps));
 }
 
-// One row-warp item of a plan's batch (q.item[k]); every thread of the CTA
-// calls it. F frames, one pass over the entries.
+// Row-warp item k of a plan's batch: a long row, eight rows of a warp each, or 32
+// tiny ones (QueuePlan's n_long, n_mid, first_tiny); every thread of the CTA calls
+// it. F frames, one pass over the entries.
 template <int MODE, typename P, int F, int U = kRowsU>
 __device__ __forceinline__ void rows_item(const QueuePlan &qp, int k, int fb, RowsRed &s_red) {
     constexpr int NA = NAcc<MODE, P>::value;
@@ -2232,7 +2233,8 @@ void run_gather(GatherTable &t, const void *d_frames, int dtype, int64_t n_pixel
     const int mode = (flags & DG_AZIMUTHAL_STD) ? kSpread : (flags & DG_ERRORS) ? kErrors
                                                                                 : kIntensity;
     // Frames per launch: 256, or fewer where the caller's fixed scratch holds
-    // the partial sums of fewer frames (the bin tiles write no partial sums).
+    // the partial sums of fewer frames (of the bin tiles, the pieces of cut tiles
+    // alone leave any; the row warps none).
     int64_t chunk = 256;
     double *partial = nullptr;
     if (scratch) {

@@ -88,15 +88,9 @@ __device__ __forceinline__ void cp_async4(void *dst, const void *src) {
     const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
-// The same with the shared-memory address as a 32-bit integer, and a 32-bit
-// shared-memory load: address arithmetic stays in 32 bits.
+// The same with the shared-memory address as a 32-bit integer.
 __device__ __forceinline__ void cp_async4_s(unsigned d, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ uint32_t lds32(unsigned a) {
-    uint32_t v;
-    asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(v) : "r"(a));
-    return v;
 }
 // A staged 4-byte pixel from its bits.
 template <typename S>

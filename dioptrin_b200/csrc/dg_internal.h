@@ -335,7 +335,7 @@ struct GatherTable {
     DeviceArray<float4> entry_raw;
     DeviceArray<double> cnt;
     DeviceArray<uint64_t> mask_words;  // scratch: per-frame masks as words (bin tiles)
-    // Bin tiles (k_gather_bins), mappings 7 and 8; see dg_gather.cu.
+    // Bin tiles (k_gather_bins), mappings 7 and 8; see dg_bins.cu.
     BinTiles bt[2];
     // Row warps (k_rows), mapping 10: per row {row, entry begin, entry end, origin
     // entry}: rw_long rows of more than kRowsLong entries, longest first (a CTA
