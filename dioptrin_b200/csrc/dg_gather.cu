@@ -1707,6 +1707,15 @@ void launch_rows(const GatherTable &t, const P *fp, int64_t n_pixels, int nf, do
     DG_CUDA(cudaGetLastError());
 }
 
+// Bin tiles offset a frame's 4-byte pixels by 32-bit byte counts. Larger frames go to
+// the row warps, which leave no partial sums either (raw sums to an entry-lane
+// mapping). 64-bit offsets in the copy loop took 1991 us against 1908 (Eiger-4M, 256
+// frames with the spread), a loop of their own beside it 1301 against 1291 (128 float
+// frames), 840 against 834 (per-frame masks).
+bool bin_tiles_reach(int dtype, int64_t n_pixels) {
+    return dtype == DG_U16 || dtype == DG_F64 || n_pixels <= int64_t(1) << 30;
+}
+
 // Launches lane mapping `variant`; returns true when the kernel wrote the
 // normalised results to oi/os/od itself (mappings 7, 8, 10), false when it left
 // partial sums for k_finalize. Those mappings need the outputs; callers without
@@ -1727,6 +1736,10 @@ bool launch_gather(GatherTable &t, int variant, const P *fp, int64_t n_pixels, i
             variant = 2;
         }
         if (variant == 7 || variant == 8) {
+            if (oi && t.rw_n_items > 0 && !bin_tiles_reach(dtype_code<P>(), n_pixels)) {
+                launch_rows<MODE, P>(t, fp, n_pixels, nf, oi, os, od, s);
+                return true;
+            }
             if (oi && t.bt[variant - 7].n_items > 0) {
                 BinCall c{};
                 c.frames = fp;
@@ -2376,8 +2389,9 @@ namespace {
 
 // Per-frame masks on a mapping-8 plan (raw sums S, N, V, C, or the normalised
 // results), and raw sums over the plan mask on a bin-tile plan: the tiles take them.
-bool bin_tiles_take_raw(const GatherTable &t, int mode, bool raw) {
-    return (mode == kRaw ? t.variant == 8 && t.entry_raw.ptr
+bool bin_tiles_take_raw(const GatherTable &t, int dtype, int64_t n_pixels, int mode, bool raw) {
+    return bin_tiles_reach(dtype, n_pixels) &&
+           (mode == kRaw ? t.variant == 8 && t.entry_raw.ptr
                          : raw && gather_variant_needs_tiles(t.variant)) &&
            t.bt[t.variant - 7].n_items > 0;
 }
@@ -2387,7 +2401,7 @@ bool launch_raw(GatherTable &t, const void *frames, int64_t n_pixels, int nf, in
                 const uint8_t *masks, int64_t mask_stride, cudaStream_t s, bool raw, double *o0,
                 double *o1, double *o2, double *o3) {
     const P *fp = static_cast<const P *>(frames);
-    if (bin_tiles_take_raw(t, mode, raw)) {
+    if (bin_tiles_take_raw(t, dtype_code<P>(), n_pixels, mode, raw)) {
         BinCall c{};
         c.frames = frames;
         c.dtype = dtype_code<P>();
@@ -2426,8 +2440,9 @@ void run_gather_raw(GatherTable &t, const void *d_frames, int dtype, int64_t n_p
     const int mode = d_masks ? kRaw : errors ? kErrors : kIntensity;
     const int64_t chunk = 256;
     // the partial sums of the mapping that runs
-    const int64_t rows = bin_tiles_take_raw(t, mode, raw) ? bin_tile_partials(t, t.variant)
-                                                          : std::max<int64_t>(1, t.n_segments);
+    const int64_t rows = bin_tiles_take_raw(t, dtype, n_pixels, mode, raw)
+                             ? bin_tile_partials(t, t.variant)
+                             : std::max<int64_t>(1, t.n_segments);
     const int64_t need = rows * n_accumulators(mode, dtype == DG_F32 || dtype == DG_F64) *
                          std::min<int64_t>(chunk, (n_frames + 31) / 32 * 32);
     if (t.partial.count < size_t(need)) t.partial.alloc(size_t(need));
